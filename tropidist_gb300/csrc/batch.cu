@@ -29,17 +29,17 @@ namespace tg {
 #define BT_THREADS FP_THREADS
 
 struct BJob {
-    int kind;                // 0 sweep, 1 fused pass, 2 one-op pass
+    int kind;                // 0 sweep, 1 fused pass, 2 one-op pass, 3 granule pass
     int plan;
     uint32_t nunits;
     uint32_t next;           // the plan's next job (BJ_NONE: the plan ends)
-    uint64_t params_off;     // SweepParams / PassParams in the parameter blob
+    uint64_t params_off;     // SweepParams / PassParams / GranParams in the parameter blob
     uint64_t src_off, dst_off;
     int bits;                // one-op pass: width of the input table
     int op_code;
     uint64_t op_a;
     uint32_t op_b;
-    uint32_t grain;          // fused pass: tiles per unit
+    uint32_t grain;          // fused or granule pass: tiles or steps per unit
 };
 
 struct BatchArgs {
@@ -107,17 +107,27 @@ __device__ void batch_single_op(const BJob &J, unsigned unit, const uint8_t *src
     }
 }
 
+// steps of a granule pass by blocks of FP_THREADS threads
+__host__ __device__ __forceinline__ uint64_t gran_steps(const GranParams &P) {
+    return (P.ncosets + FP_THREADS - 1) >> FP_TBITS;
+}
+
 // one unit of a job by the whole block: TC = three 64 KB tile buffers, PRM = parameter copy
 __device__ void run_unit(const BJob &J, unsigned unit, uint8_t *arena, const uint8_t *params, uint4 *TC, uint4 *PRM) {
     const uint8_t *src = arena + J.src_off;
     uint8_t *dst = arena + J.dst_off;
-    if (J.kind == 0 || J.kind == 1) {
-        const size_t psize = J.kind == 0 ? sizeof(SweepParams) : sizeof(PassParams);
+    if (J.kind != 2) {
+        const size_t psize = J.kind == 0 ? sizeof(SweepParams) : J.kind == 1 ? sizeof(PassParams) : sizeof(GranParams);
         const uint4 *g = reinterpret_cast<const uint4 *>(params + J.params_off);
         for (uint32_t i = threadIdx.x; i < (psize + 15) / 16; i += blockDim.x) PRM[i] = __ldcg(g + i);
         __syncthreads();
         if (J.kind == 0) {
             sweep_body<uint8_t>(*reinterpret_cast<const SweepParams *>(PRM), src, dst, TC);
+        } else if (J.kind == 3) {
+            const GranParams &P = *reinterpret_cast<const GranParams *>(PRM);
+            const uint32_t n = (uint32_t)gran_steps(P), s0 = unit * J.grain, s1 = min(s0 + J.grain, n);
+            for (uint32_t s = s0; s < s1; s++)
+                gran_step<1, FP_TBITS, false>(P, s, reinterpret_cast<const uint32_t *>(src), reinterpret_cast<uint32_t *>(dst));
         } else {
             const PassParams &P = *reinterpret_cast<const PassParams *>(PRM);
             const uint64_t t0 = (uint64_t)unit * J.grain;
@@ -221,7 +231,35 @@ static uint32_t pass_grain(uint64_t nt) {
     return (uint32_t)std::min<uint64_t>(nt, std::max<uint64_t>(16, (nt + sm_count() - 1) / sm_count()));
 }
 
-static_assert(sizeof(SweepParams) <= 4096 && sizeof(PassParams) <= 4096, "job parameters exceed their 4 KB copy");
+static_assert(sizeof(SweepParams) <= 4096 && sizeof(PassParams) <= 4096 && sizeof(GranParams) <= 4096, "job parameters exceed their 4 KB copy");
+// the pass-specific part of a segment's job (kind, units, one-op fields); returns its parameter record
+static const void *fill_job(const Seg &S, BJob &J, size_t &bytes) {
+    bytes = 0;
+    if (S.kind == 0) {
+        J.kind = 0;
+        J.nunits = 1;
+        bytes = sizeof(SweepParams);
+        return &S.sp;
+    }
+    if (S.kind == 2) {
+        J.kind = 2;
+        J.bits = S.w_in;
+        J.op_code = S.op_code;
+        J.op_a = S.op_a;
+        J.op_b = S.op_b;
+        const uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)1 << S.w_in) >> 4);
+        J.nunits = (uint32_t)((chunks + BJ_UNIT_CHUNKS - 1) / BJ_UNIT_CHUNKS);
+        return nullptr;
+    }
+    // large units amortise the per-unit overhead; concurrency comes from the other plans
+    J.kind = S.kind == 4 ? 3 : 1;
+    const uint64_t nt = S.kind == 4 ? gran_steps(S.gp) : pass_units(S.pp);
+    J.grain = pass_grain(nt);
+    J.nunits = (uint32_t)((nt + J.grain - 1) / J.grain);
+    bytes = S.kind == 4 ? sizeof(GranParams) : sizeof(PassParams);
+    return S.kind == 4 ? (const void *)&S.gp : (const void *)&S.pp;
+}
+
 static_assert(sizeof(BJob) % 16 == 0, "job descriptors are read as 16-byte words");
 
 static bool g_batch_attr = false;
@@ -459,29 +497,12 @@ void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, in
                 J.next = BJ_NONE;
                 J.src_off = cur ? b : a;
                 J.dst_off = cur ? a : b;
-                if (S.kind == 0) {
-                    J.kind = 0;
-                    J.nunits = 1;
+                size_t bytes;
+                const void *rec = fill_job(S, J, bytes);
+                if (bytes) {
                     J.params_off = align_up(B->params.size(), 16);
-                    B->params.resize(J.params_off + sizeof(SweepParams));
-                    memcpy(B->params.data() + J.params_off, &S.sp, sizeof(SweepParams));
-                } else if (S.kind == 1) {
-                    J.kind = 1;
-                    // large units amortise the per-unit overhead; concurrency comes from the other plans
-                    const uint64_t nt = pass_units(S.pp);
-                    J.grain = pass_grain(nt);
-                    J.nunits = (uint32_t)((nt + J.grain - 1) / J.grain);
-                    J.params_off = align_up(B->params.size(), 16);
-                    B->params.resize(J.params_off + sizeof(PassParams));
-                    memcpy(B->params.data() + J.params_off, &S.pp, sizeof(PassParams));
-                } else {
-                    J.kind = 2;
-                    J.bits = S.w_in;
-                    J.op_code = S.op_code;
-                    J.op_a = S.op_a;
-                    J.op_b = S.op_b;
-                    const uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)1 << S.w_in) >> 4);
-                    J.nunits = (uint32_t)((chunks + BJ_UNIT_CHUNKS - 1) / BJ_UNIT_CHUNKS);
+                    B->params.resize(J.params_off + bytes);
+                    memcpy(B->params.data() + J.params_off, rec, bytes);
                 }
                 B->units += J.nunits;
                 const unsigned idx = (unsigned)B->jobs.size();
@@ -751,7 +772,9 @@ static int server_submit(Server &S, const DensePlan &P) {
     R.arena_bytes = 2 * tb;
     if (!S.arena_a.take(R.arena_bytes, R.arena_off)) return TG_ERR_NOMEM;
     for (const Seg &G : P.segs) {
-        const size_t n = G.kind == 0 ? sizeof(SweepParams) : G.kind == 1 ? sizeof(PassParams) : 0;
+        BJob J;
+        size_t n;
+        fill_job(G, J, n);
         if (n) prm.resize(align_up(prm.size(), 16) + n);
     }
     R.prm_bytes = std::max<size_t>(16, prm.size());
@@ -778,30 +801,13 @@ static int server_submit(Server &S, const DensePlan &P) {
         J.next = k + 1 < P.segs.size() ? (unsigned)(R.job0 + k + 1) : BJ_NONE;
         J.src_off = cur ? b : a;
         J.dst_off = cur ? a : b;
-        if (G.kind == 0) {
-            J.kind = 0;
-            J.nunits = 1;
+        size_t bytes;
+        const void *rec = fill_job(G, J, bytes);
+        if (bytes) {
             poff = align_up(poff, 16);
-            memcpy(prm.data() + poff, &G.sp, sizeof(SweepParams));
+            memcpy(prm.data() + poff, rec, bytes);
             J.params_off = R.prm_off + poff;
-            poff += sizeof(SweepParams);
-        } else if (G.kind == 1) {
-            J.kind = 1;
-            const uint64_t nt = pass_units(G.pp);
-            J.grain = pass_grain(nt);
-            J.nunits = (uint32_t)((nt + J.grain - 1) / J.grain);
-            poff = align_up(poff, 16);
-            memcpy(prm.data() + poff, &G.pp, sizeof(PassParams));
-            J.params_off = R.prm_off + poff;
-            poff += sizeof(PassParams);
-        } else {
-            J.kind = 2;
-            J.bits = G.w_in;
-            J.op_code = G.op_code;
-            J.op_a = G.op_a;
-            J.op_b = G.op_b;
-            const uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)1 << G.w_in) >> 4);
-            J.nunits = (uint32_t)((chunks + BJ_UNIT_CHUNKS - 1) / BJ_UNIT_CHUNKS);
+            poff += bytes;
         }
         cur ^= 1;
     }

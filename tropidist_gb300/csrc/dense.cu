@@ -350,6 +350,11 @@ static bool g_relayout = true;                       // uint8 layout planning be
 static bool g_cosets = true;                         // coset-streaming form of one-group uint8 passes
 static int g_span = 3, g_span_sel = 2;               // streaming passes: update span (4: lane dimension),
                                                      // span when an in-chunk row closes in the pass
+// Granule passes take the wide tables of both entry sizes unless a knob asks for another form: a tile
+// narrower than the 2^12 bytes that a warp of the granule pass holds, or a streaming span other than
+// the default.  One sweep, the other forms against granule passes: uint8 31 bits 48.4 / 19.2 ms, 26 bits
+// 4.74 / 2.15 ms; uint16 27 bits 10.9 / 1.73 ms.
+static bool use_gran(int eb) { return (eb == 1 ? g_dmax8 >= 12 : g_dmax16 >= 11) && g_span == 3 && g_span_sel == 2; }
 
 // Groups of the pass's updates whose chunk masks (mask >> 4) span <= 3 dimensions, every update
 // in a group (the in-chunk part of a mask is free in the register form; see fused_u8.cuh).  Also
@@ -693,6 +698,7 @@ struct RowInfo {
     std::vector<std::vector<int>> upd_rows;     // per op: rows of an update
     std::vector<int> sel_row, exp_row;          // per op: row closed / opened (-1)
     std::vector<std::vector<int64_t>> uses;     // per row: ops that update or close it (ascending)
+    std::vector<int64_t> close_op;              // per row: the op that closes it (INT64_MAX: none does)
     int64_t next_use(int row, int64_t after) const {
         const auto &u = uses[row];
         auto it = std::lower_bound(u.begin(), u.end(), after);
@@ -726,8 +732,14 @@ static void row_info(const std::vector<HostOp> &hops, RowInfo &R, int w0 = 0) {
             canon.erase(canon.begin() + o.a);
         }
     }
+    R.close_op.assign(R.uses.size(), INT64_MAX);
+    for (int64_t i = 0; i < n; i++)
+        if (R.sel_row[i] >= 0) R.close_op[R.sel_row[i]] = i;
 }
 
+}  // namespace tg
+#include "gran_sched.h"
+namespace tg {
 
 int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ckpts, int64_t nckpt,
                      DensePlan &P, int w_start, bool open_end, SegHook on_seg, void *hook_ctx) {
@@ -743,6 +755,7 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
     const int DMAX = eb == 1 ? g_dmax8 : g_dmax16;
     const int SWB = eb == 1 ? g_sweep_bits8 : g_sweep_bits16;
     const bool relayout = eb == 1 && g_relayout;
+    const bool gran = use_gran(eb);
     P.eb = eb;
     P.peak_bits = peak;
     P.nops = nops;
@@ -955,12 +968,24 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
         const int64_t limit = next_ckpt[i];
         Seg S;
         S.w_in = w_in;
-        if (sweep_next(w_in, i) && phys != canon) {
-            e = build_pass(i, i, {}, true, S);
-            if (e) return e;
+        const int64_t i_seg = i;
+        int gran_upd = 0;
+        int64_t gran_end = -1;
+        if (gran && !sweep_next(w_in, i)) {
+            gran_end = build_gran(hops, RI, i, limit, eb, canon, phys, S.gp, gran_upd);
+            if (gran_end == -2) return set_error(TG_ERR_STATE, "granule pass maps disagree");
+        }
+        if (gran_end >= 0) {
+            S.kind = 4;
+            S.w_out = (int)canon.size();
+            S.op_end = gran_end;
+            P.n_updates += gran_upd;
+            P.pass_bytes += (double)eb * ((1ull << w_in) + (1ull << S.w_out));
+            i = gran_end;
         } else if (sweep_next(w_in, i)) {
             SweepParams &sp = S.sp;
             memset(&sp, 0, sizeof(sp));
+            for (int q = 0; q < w_in && q < 20; q++) sp.in_pos[q] = (uint8_t)index_of(canon, phys[q]);
             sp.w_in = w_in;
             sp.has_in = (i > 0 || w_start > 0) ? 1 : 0;
             sp.max_bits = SWB;
@@ -984,6 +1009,10 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
             }
             if (j == i) return set_error(TG_ERR_STATE, "scheduler made no progress");
             phys = canon;
+            // before a granule pass: the rows that live longest take the lowest positions
+            if (gran && j < nops && !is_ckpt[j])
+                std::stable_sort(phys.begin(), phys.end(), [&](int x, int y) { return RI.close_op[x] > RI.close_op[y]; });
+            for (int q = 0; q < w && q < 20; q++) sp.out_pos[q] = (uint8_t)index_of(canon, phys[q]);
             S.kind = 0;
             S.w_out = w;
             S.op_end = j;
@@ -1089,7 +1118,8 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
         buf ^= 1;
         // checkpoints and the end of a plan that ends with a table are in canonical order
         const bool end_table = open_end && S.op_end == nops;
-        if ((is_ckpt[S.op_end] || end_table) && phys != canon) {
+        const bool at_ckpt = is_ckpt[S.op_end] && S.op_end > i_seg;    // not a pass that only moved rows
+        if ((at_ckpt || end_table) && phys != canon) {
             P.segs.push_back(S);
             if (on_seg && (e = on_seg(P.segs.back(), hook_ctx))) return e;
             Seg R;
@@ -1099,7 +1129,7 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
             S = R;
             buf ^= 1;
         }
-        if (is_ckpt[S.op_end]) {
+        if (at_ckpt) {
             if (phys != canon) return set_error(TG_ERR_STATE, "checkpoint with a non-canonical layout");
             for (size_t c = 0; c < P.ckpt_ops.size(); c++)
                 if (P.ckpt_ops[c] == S.op_end) { S.ckpt = (int)c; break; }
@@ -1167,6 +1197,9 @@ static int launch_seg(const Seg &S, E *const bufs[2], int &cur, void **ckpt_bufs
     } else if (S.kind == 0) {
         size_t sm = 2 * ((size_t)1 << S.sp.max_bits) * sizeof(E);
         k_sweep_smem<E><<<1, 512, sm, st>>>(S.sp, src, dst);
+    } else if (S.kind == 4) {
+        e = launch_gran(S.gp, sizeof(E), src, dst, st);
+        if (e) return e;
     } else {
         size_t sm = ((size_t)1 << S.pp.d) * sizeof(E);
         if (sizeof(E) == 1 && S.pp.stream) {
@@ -1422,10 +1455,18 @@ static void emulate_plan(const DensePlan &P, E *a, E *b, void **ckpt) {
                     dst[k] = src[((k ^ lo) << 1) | lo | ((uint64_t)S.op_b << pos)];
                 }
             }
+        } else if (S.kind == 4) {
+            emulate_gran<E>(S.gp, src, dst);
         } else if (S.kind == 0) {
             std::vector<E> T;
-            if (S.sp.has_in) T.assign(src, src + (1ull << S.sp.w_in));
-            else T.assign(1, 0);
+            auto canon_index = [](size_t x, const uint8_t *pos, int bits) {
+                size_t s = 0;
+                for (int q = 0; q < bits; q++) s |= ((x >> q) & 1u) << pos[q];
+                return s;
+            };
+            T.assign(S.sp.has_in ? (size_t)1 << S.sp.w_in : 1, 0);
+            if (S.sp.has_in)
+                for (size_t x = 0; x < T.size(); x++) T[canon_index(x, S.sp.in_pos, S.sp.w_in)] = src[x];
             for (int i = 0; i < S.sp.nops; i++) {
                 uint32_t op = S.sp.ops[i], code = op >> 30;
                 size_t n = T.size();
@@ -1452,7 +1493,7 @@ static void emulate_plan(const DensePlan &P, E *a, E *b, void **ckpt) {
                     T.swap(U);
                 }
             }
-            std::copy(T.begin(), T.end(), dst);
+            for (size_t x = 0; x < T.size(); x++) dst[x] = T[canon_index(x, S.sp.out_pos, S.w_out)];
         } else {
             const PassParams &pp = S.pp;
             std::vector<E> T((size_t)1 << pp.d);
@@ -1806,7 +1847,11 @@ int tg_dense_plan_segments(void *plan, int64_t *out, int64_t maxseg) {
         o[2] = S.w_out;
         o[3] = S.op_end;
         o[4] = S.kind == 1 ? S.pp.d : S.kind == 0 ? S.sp.max_bits : -1;
-        o[5] = S.kind == 1 ? S.pp.nupd : S.kind == 0 ? S.sp.nops : (S.op_code == 1);
+        o[5] = S.kind == 1 ? S.pp.nupd : S.kind == 0 ? S.sp.nops : S.kind == 2 ? (S.op_code == 1) : 0;
+        if (S.kind == 4) {
+            o[4] = GP_SLOTS;
+            for (int u = 0; u < S.gp.nops; u++) o[5] += S.gp.ops[u].code <= GC_A || S.gp.ops[u].code >= GC_I1;
+        }
         if (S.kind == 1 && S.pp.stream) {
             int ws = 0;
             for (int x = 0; x < 8; x++) ws |= S.pp.s_wsw[x] != 0;
@@ -1844,8 +1889,8 @@ int tg_dense_execute(void *plan, void *buf_a, void *buf_b, void **ckpt_bufs, voi
 }
 
 int tg_dense_execute_timed(void *plan, void *buf_a, void *buf_b, void *stream, double *out, int nout) {
-    // out: per segment kind (0 sweep, 1 fused tile pass, 2 one-op pass, 3 coset-streaming pass):
-    // launches, total ms, bytes
+    // out: per segment kind (0 sweep, 1 fused tile pass, 2 one-op pass, 3 coset-streaming pass,
+    // 4 granule pass): launches, total ms, bytes
     if (!plan || !buf_a || !buf_b || !out) return set_error(TG_ERR_ARG, "null argument");
     const DensePlan &P = *static_cast<DensePlan *>(plan);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1857,7 +1902,7 @@ int tg_dense_execute_timed(void *plan, void *buf_a, void *buf_b, void *stream, d
     if (P.segs.empty()) return TG_OK;
     e = cuda_check(cudaEventSynchronize(g_events[2 * P.segs.size() - 1]), "event sync");
     if (e) return e;
-    double acc[12] = {0};
+    double acc[15] = {0};
     DensePlan &PM = *static_cast<DensePlan *>(plan);
     PM.seg_ms.assign(P.segs.size(), 0.f);
     for (size_t k = 0; k < P.segs.size(); k++) {
@@ -1872,7 +1917,7 @@ int tg_dense_execute_timed(void *plan, void *buf_a, void *buf_b, void *stream, d
                                    : (double)P.eb * ((1ull << S.w_in) + (1ull << S.w_out));
         acc[3 * kk + 2] += bytes;
     }
-    for (int k = 0; k < nout && k < 12; k++) out[k] = acc[k];
+    for (int k = 0; k < nout && k < 15; k++) out[k] = acc[k];
     return TG_OK;
 }
 

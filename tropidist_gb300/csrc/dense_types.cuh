@@ -4,6 +4,7 @@
 #pragma once
 #include "tg_common.cuh"
 #include "fused_u8.cuh"
+#include "gran.cuh"
 
 #include <cstring>
 #include <vector>
@@ -56,8 +57,16 @@ struct SweepParams {
     int w_in;             // width of the input table (0: start from {0: 0})
     int max_bits;         // shared-memory capacity per buffer (entries = 2^max_bits)
     int has_in;
+    uint8_t in_pos[20], out_pos[20];   // physical bit q of the input / output table holds canonical bit [q]
     uint32_t ops[SW_MAXOPS];
 };
+
+// canonical index of physical index x of a table of `bits` bits
+__device__ __forceinline__ uint32_t sweep_index(uint32_t x, const uint8_t *pos, int lo, int bits) {
+    uint32_t s = 0;
+    for (int q = lo; q < bits; q++) s |= ((x >> (q - lo)) & 1u) << pos[q];
+    return s;
+}
 
 // a whole run of ops on a table held in shared memory (smem_raw: 2 x 2^max_bits entries), all
 // threads of the block; has_in: the input table is read from `in`, else the table starts as {0: 0}
@@ -69,8 +78,22 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P, const E *__rest
     E *S = T + (1u << P.max_bits);
     int bits = P.w_in;
     uint32_t n = 1u << bits;
-    if (P.has_in) {
-        for (uint32_t s = threadIdx.x; s < n; s += blockDim.x) T[s] = __ldcg(in + s);
+    if (P.has_in && bits >= CB) {
+        // 16-byte loads in physical order, entries to their canonical places
+        for (uint32_t c = threadIdx.x; c < (n >> CB); c += blockDim.x) {
+            const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(in) + c);
+            const uint32_t s = sweep_index(c, P.in_pos, CB, bits);
+            const E *e = reinterpret_cast<const E *>(&v);
+#pragma unroll
+            for (uint32_t q = 0; q < (1u << CB); q++) {
+                uint32_t o = s;
+#pragma unroll
+                for (int b = 0; b < CB; b++) o |= ((q >> b) & 1u) << P.in_pos[b];
+                T[o] = e[q];
+            }
+        }
+    } else if (P.has_in) {
+        for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) T[sweep_index(x, P.in_pos, 0, bits)] = __ldcg(in + x);
     } else if (threadIdx.x == 0) {
         T[0] = 0;
     }
@@ -103,7 +126,23 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P, const E *__rest
         }
         __syncthreads();
     }
-    for (uint32_t s = threadIdx.x; s < n; s += blockDim.x) out[s] = T[s];
+    if (bits >= CB) {
+        for (uint32_t c = threadIdx.x; c < (n >> CB); c += blockDim.x) {
+            uint4 v;
+            E *e = reinterpret_cast<E *>(&v);
+            const uint32_t s = sweep_index(c, P.out_pos, CB, bits);
+#pragma unroll
+            for (uint32_t q = 0; q < (1u << CB); q++) {
+                uint32_t o = s;
+#pragma unroll
+                for (int b = 0; b < CB; b++) o |= ((q >> b) & 1u) << P.out_pos[b];
+                e[q] = T[o];
+            }
+            *(reinterpret_cast<uint4 *>(out) + c) = v;
+        }
+    } else {
+        for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) out[x] = T[sweep_index(x, P.out_pos, 0, bits)];
+    }
 }
 
 // ------------------------------------------------------------------ fused tile pass (wide tables)
@@ -191,7 +230,7 @@ __device__ __forceinline__ uint32_t pdep_w32(uint32_t x, const uint32_t *wt, int
 struct HostOp { int code; uint64_t a; int64_t b; };
 
 struct Seg {
-    int kind;               // 0 sweep in shared memory, 1 fused pass, 2 one op out of place
+    int kind;               // 0 sweep in shared memory, 1 fused pass, 2 one op out of place, 4 granule pass
     int op_code = 0;
     uint64_t op_a = 0;
     uint32_t op_b = 0;
@@ -199,6 +238,7 @@ struct Seg {
     int64_t op_end;         // ops done after this segment
     SweepParams sp;
     PassParams pp;
+    GranParams gp;
     int ckpt = -1;          // index of a checkpoint written after this segment
 };
 
@@ -657,5 +697,7 @@ using SegHook = int (*)(const Seg &S, void *ctx);
 int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ckpts, int64_t nckpt, DensePlan &P,
                      int w_start = 0, bool open_end = false, SegHook on_seg = nullptr, void *hook_ctx = nullptr);
 int set_dense_attrs();
+// one granule pass (gran.cu): tables of eb-byte entries
+int launch_gran(const GranParams &P, int eb, const void *in, void *out, cudaStream_t st);
 
 }  // namespace tg
