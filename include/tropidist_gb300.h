@@ -163,6 +163,11 @@ int tg_sp_bound_data_wide(int N, int nrows, const int64_t *row_ptr, const int32_
 int tg_sp_walk(int nsteps, const int64_t *spec, const uint64_t *masks, const int64_t *weights, int stride, int K,
                const void *A0, uint64_t n0, const void *H0, int lg0, void *scratch, uint64_t cap_n, void *arena,
                uint64_t arena_bytes, int64_t *out, void *join_results, int64_t *need, void *counters, void *stream);
+/* traceback through a run of steps in one launch (the lookups of the reference's traceback): rows DEVICE
+ * int64 [nsteps][5] (index of the table before the step, its lg, closing bits, column, weight; the last
+ * step first), from state s of value v; state DEVICE int64 [3]: state, value, steps done (fewer than
+ * nsteps where no table holds the path); used DEVICE uint8 [nsteps]: 1 where the column was used */
+int tg_sp_trace(int nsteps, const void *rows, uint64_t s, int v, void *state, void *used, void *stream);
 /* replaces sp_hist (cdist/sparse_dp.c:239-242): hist is a device uint64[256] */
 int tg_sp_hist(const void *A, uint64_t n, void *hist, void *stream);
 
@@ -195,6 +200,10 @@ int tg_spw_join(int W, const void *fkeys, const void *fvals, uint64_t nf, uint64
 int tg_spw_lookup(int W, const void *H, int lg, const void *keys, uint64_t stride, const void *q, uint64_t m,
                   void *out, void *stream);
 
+/* tg_sp_trace on wide states: rows DEVICE int64 [nsteps][5 + 2 W] (index, lg, keys, key stride, weight,
+ * closing bits, column), state DEVICE uint64 [W + 2] in and out (state, value, steps done) */
+int tg_spw_trace(int W, int nsteps, const void *rows, void *state, void *used, void *stream);
+
 /* A leg of column steps on wide states in one call, with the table sizes kept on the device and
  * one host read at the end (the multi-word counterpart of tg_sp_walk; the per-step rule of
  * cdist/sparse_dp.py:338-403).  steps HOST int64 [nsteps][13] = cap, keep_below, w, trunc (< 0:
@@ -209,7 +218,7 @@ int tg_spw_lookup(int W, const void *H, int lg, const void *keys, uint64_t strid
  * total (all ones: none), forward value, forward key words.  Returns nsteps, or 0 with need[0]
  * (states per table) or need[1] (arena bytes) set: run the leg again with more room. */
 int64_t tg_spw_walk_scratch_bytes(int W, uint64_t cap, int nsteps);
-/* tables of at most limit / 2 states are stepped by one block per launch (default 512; 0: never);
+/* tables of at most limit / 2 states are stepped by one block per launch (default 4096; 0: never);
  * returns the previous limit (a negative argument only reads it) */
 int64_t tg_spw_set_small_limit(int64_t limit);
 int tg_spw_walk(int W, int nsteps, const int64_t *steps, const uint64_t *words, const uint64_t *masks,

@@ -41,16 +41,22 @@ struct BoundParams {
     int64_t w[SP_MAXCLS];
 };
 
-// ceil((extra + sum_c w_c * |(key ^ tmask) & mask_c|) / QW)   (cdist/sparse_dp.py:208-217)
-__device__ __forceinline__ int64_t sp_hbound(const BoundParams &b, uint64_t key) {
+// v + ceil((extra + sum_c w_c * |(key ^ tmask) & mask_c|) / QW) <= K   (cdist/sparse_dp.py:208-217),
+// multiplied out (a 64-bit division costs more than the rest of the test)
+__device__ __forceinline__ bool sp_keep(const BoundParams &b, uint64_t key, uint32_t v) {
+    if (!b.on) return true;
     const uint64_t u = key ^ b.tmask;
     int64_t tot = b.extra;
     for (int c = 0; c < b.ncls; c++) tot += b.w[c] * (int64_t)__popcll(u & b.mask[c]);
-    return (tot + SP_QW - 1) / SP_QW;
+    return tot <= ((int64_t)b.K - (int64_t)v) * SP_QW;
 }
 
-__device__ __forceinline__ bool sp_keep(const BoundParams &b, uint64_t key, uint32_t v) {
-    return !b.on || (int64_t)v + sp_hbound(b, key) <= (int64_t)b.K;
+// position claimed in a list by the lanes that want one (all lanes of the warp call): one atomic a warp
+__device__ __forceinline__ unsigned long long sp_claim(unsigned long long *ctr, bool want) {
+    const unsigned bal = __ballot_sync(0xffffffffu, want), lane = threadIdx.x & 31u;
+    unsigned long long base = 0;
+    if (lane == 0 && bal) base = atomicAdd(ctr, (unsigned long long)__popc(bal));
+    return __shfl_sync(0xffffffffu, base, 0) + __popc(bal & ((1u << lane) - 1u));
 }
 
 __device__ __forceinline__ uint32_t sp_slot(uint64_t key, int lg) {
@@ -222,6 +228,42 @@ __global__ void k_sp_lookup(const unsigned long long *H, int lg, const unsigned 
         vals[i] = (uint8_t)sp_lookup(H, lg, keys[i] & SP_KEYMASK);
 }
 
+// The traceback through a run of steps, one warp: step i (rows [H, lg, closing bits, column, weight],
+// the last step of the sweep first) used its column unless the table before it holds the state
+// (closing bits restored) with the same value.  The state's and its partner's lookups run side by side
+// on two lanes, the next step's row is read meanwhile.  A dependent chain of two index probes a step
+// (about 1.3 us), where a lookup call per step cost a launch, two copies and a synchronisation
+// (100 us).  used[i]: 1 if the column was used; state: [0] state, [1] value, [2] steps done.
+__global__ void k_sp_trace(const int64_t *__restrict__ rows, int n, uint64_t s, int v, uint8_t *used, int64_t *state) {
+    const unsigned lane = threadIdx.x;
+    int64_t nx[5] = {0, 0, 0, 0, 0};
+    if (n)
+        for (int q = 0; q < 5; q++) nx[q] = rows[q];
+    int i = 0;
+    for (; i < n; i++) {
+        int64_t r[5];
+        for (int q = 0; q < 5; q++) r[q] = nx[q];
+        if (i + 1 < n)
+            for (int q = 0; q < 5; q++) nx[q] = rows[5 * (size_t)(i + 1) + q];
+        const uint64_t mid = s | (uint64_t)r[2], col = (uint64_t)r[3];
+        uint32_t val = 255u;
+        if (lane < 2)
+            val = sp_lookup(reinterpret_cast<const unsigned long long *>((uintptr_t)r[0]), (int)r[1],
+                            (lane ? mid ^ col : mid) & SP_KEYMASK);
+        const int without = (int)__shfl_sync(0xffffffffu, val, 0), with_col = (int)__shfl_sync(0xffffffffu, val, 1);
+        const bool take = without != v;
+        if (take && (!col || with_col != v - (int)r[4])) break;
+        s = take ? mid ^ col : mid;
+        if (take) v -= (int)r[4];
+        if (lane == 0) used[i] = take ? 1 : 0;
+    }
+    if (lane == 0) {
+        state[0] = (int64_t)s;
+        state[1] = v;
+        state[2] = i;
+    }
+}
+
 // value histogram of an array (hist[256], values 0..255)
 __global__ void k_sp_hist(const unsigned long long *__restrict__ A, uint64_t n, unsigned long long *hist) {
     __shared__ unsigned int loc[256];
@@ -284,7 +326,11 @@ __global__ void k_sp_join_acc(const unsigned long long *__restrict__ F, uint64_t
 }
 
 // ---- small tables: one block runs many steps per launch (no host round trip per column)
-#define SPW_SMALL_MAX 4096              // states per table in the one-block walk
+// One block steps tables of up to SPW_SMALL_MAX / 2 states (and half the scratch's room): at 8192 states
+// a step takes it 8 rounds of L2 latency, less than the three launches and the synchronisation of a step
+// by separate kernels.
+#define SPW_SMALL_MAX 16384
+#define SPW_SMALL_MIN 256               // scratch of fewer states: separate kernels only
 #define SPW_SMALL_THREADS 1024
 
 struct WalkSmall {
@@ -292,6 +338,7 @@ struct WalkSmall {
     const uint64_t *masks;
     const int64_t *weights;
     int stride, K, i0, nsteps;
+    uint64_t limit;                     // largest 2 n stepped
     const unsigned long long *A0, *H0;  // the table before step i0
     uint64_t n0;
     int lg0, slot0;                     // slot0: scratch slot of that table (-1: outside the scratch)
@@ -303,389 +350,403 @@ struct WalkSmall {
     unsigned long long *state;          // out: [0] next step, [1] slot, [2] n, [3] lg, [4] arena used, [5] stop reason
 };
 
-// ---- tiny tables: the same steps with the working tables in shared memory
-// The three scratch slots (states and index), the changed list and a copy of the join table live
-// in shared memory, so a step touches global memory only for its outputs, kept tables and large
-// join tables; the next step's rows are fetched while the current step runs.  It takes tables of at
-// most SPW_TINY_N / 2 states with an index of at most 2^SPW_TINY_LG slots and stops (reason 1) when
-// a step would need more; the table it ends with is written back to its global scratch slot.
-#define SPW_TINY_N 1024
-#define SPW_TINY_LG 12
-#define SPW_TINY_THREADS 512
-#define SPW_TINY_SMEM (8 * (3 * SPW_TINY_N + 3 * (1 << SPW_TINY_LG) + SPW_TINY_N + (1 << SPW_TINY_LG)))
+// index bits of the shared-memory tables: load at most 1/2 for m states
+__host__ __device__ static int lg_tiny(uint64_t m) {
+    int b = 6;
+    while ((1ull << b) < 2 * m) b++;
+    return b;
+}
+
+// ---- tables that fit shared memory: the same steps with the old table, the new one and the changed list
+// there, so that index probes and claims are shared-memory atomics: from the global scratch one SM's
+// random L2 atomics bound the step (25 us a step at 1000 states; 13 us here, host included).  It takes tables of at most SPW_TINY_N / 2
+// states and stops (reason 1) when a step would need more.  The next step's row is fetched during this
+// one.  A kept table is a plain copy of its states and of the working index (load 1/4 to 1/2), unless
+// that index is more than twice what the table needs.  The truncated table of a cut takes the old
+// table's place, free by then.  The table it ends with is written to a global scratch slot.
+#define SPW_TINY_N 4096
+#define SPW_TINY_LG 13
+#define SPW_TINY_THREADS 1024
+#define SPW_TINY_SMEM (8 * (2 * SPW_TINY_N + 2 * (1 << SPW_TINY_LG) + SPW_TINY_N / 2))
 
 __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_constant__ WalkSmall P) {
     extern __shared__ unsigned long long sm_tiny[];
     auto sA = [&](int k) { return sm_tiny + k * SPW_TINY_N; };
-    auto sH = [&](int k) { return sm_tiny + 3 * SPW_TINY_N + k * (1 << SPW_TINY_LG); };
-    unsigned long long *sCH = sm_tiny + 3 * SPW_TINY_N + 3 * (1 << SPW_TINY_LG);
-    unsigned long long *sJ = sCH + SPW_TINY_N;
-    __shared__ unsigned long long c_ch, c_out, c_tr, c_flag;
-    __shared__ BoundParams B[2];
-    __shared__ int64_t F[2][SPW_FIELDS];
-    __shared__ const unsigned long long *j_cached;
+    auto sH = [&](int k) { return sm_tiny + 2 * SPW_TINY_N + k * (1 << SPW_TINY_LG); };
+    unsigned long long *sCH = sm_tiny + 2 * SPW_TINY_N + 2 * (1 << SPW_TINY_LG);
+    __shared__ unsigned long long c_cnt[2][3], c_flag;   // per step parity: changed, states, truncated
+    __shared__ BoundParams B2[2];
+    __shared__ int64_t F2[2][SPW_FIELDS];
     const unsigned tid = threadIdx.x, NT = blockDim.x;
-    int cur = P.slot0;
-    int sc = cur >= 0 ? cur : 2;          // shared slot of the current table (an outside table goes to 2)
+    const uint64_t limit = P.limit < SPW_TINY_N ? P.limit : SPW_TINY_N;
+    int sl = 0;                                          // shared slot of the current table
     uint64_t n = P.n0;
-    int lg = P.lg0;
+    int lg = lg_tiny(n);
     uint64_t used = P.used0;
     int i = P.i0, reason = 0;
-    // the table before step i0, and the rows of step i0
-    for (uint64_t k = tid; k < n; k += NT) sA(sc)[k] = P.A0[k];
-    for (uint64_t k = tid; k < (1ull << lg); k += NT) sH(sc)[k] = P.H0[k];
-    auto load_rows = [&](int step, int buf) {
+    auto load_row = [&](int step, int b) {
         const int64_t *f = P.spec + (size_t)SPW_FIELDS * step;
-        if (tid < SPW_FIELDS) F[buf][tid] = f[tid];
-        const int nc = (int)f[SW_NCLS];
-        for (int c = tid; c < nc && c < SP_MAXCLS; c += NT) {
-            B[buf].mask[c] = P.masks[(size_t)P.stride * step + c];
-            B[buf].w[c] = P.weights[(size_t)P.stride * step + c];
-        }
+        if (tid < SPW_FIELDS) F2[b][tid] = f[tid];
+        BoundParams &B = B2[b];
         if (tid == 0) {
-            B[buf].on = (int)f[SW_USEH];
-            B[buf].ncls = nc;
-            B[buf].K = P.K;
-            B[buf].extra = f[SW_EXTRA];
-            B[buf].tmask = (uint64_t)f[SW_TMASK];
-        }
-    };
-    if (i < P.nsteps) load_rows(i, i & 1);
-    if (tid == 0) { c_ch = c_out = c_tr = c_flag = 0; j_cached = nullptr; }
-    __syncthreads();
-    for (; i < P.nsteps; i++) {
-        const int b = i & 1;
-        const int64_t *f = F[b];
-        if (2 * n > SPW_TINY_N) { reason = 1; break; }
-        int os = 0;
-        while (os == cur) os++;
-        const int lgn = lg_for(2 * n);
-        const uint64_t capn = 1ull << lgn;
-        unsigned long long *H = sH(os), *A = sA(os);
-        for (uint64_t k = tid; k < capn; k += NT) H[k] = SP_EMPTY;
-        // the next step's rows: loads issued now, stored at the end of the step
-        int64_t pf = 0;
-        uint64_t pm = 0;
-        int64_t pw = 0;
-        const bool more = i + 1 < P.nsteps;
-        if (more) {
-            const int64_t *fn = P.spec + (size_t)SPW_FIELDS * (i + 1);
-            if (tid < SPW_FIELDS) pf = fn[tid];
-            if (tid >= 32 && tid < 32 + (unsigned)SP_MAXCLS && (int)(tid - 32) < P.stride) {
-                pm = P.masks[(size_t)P.stride * (i + 1) + (tid - 32)];
-                pw = P.weights[(size_t)P.stride * (i + 1) + (tid - 32)];
-            }
-        }
-        // a join table small enough is copied once and then probed in shared memory
-        const unsigned long long *jG = reinterpret_cast<const unsigned long long *>((uintptr_t)f[SW_JTAB]);
-        const int jlg = (int)f[SW_JLG];
-        const bool jS = jG && jlg <= SPW_TINY_LG;
-        if (jS && j_cached != jG)
-            for (uint64_t k = tid; k < (1ull << jlg); k += NT) sJ[k] = jG[k];
-        __syncthreads();
-        if (tid == 0 && jS) j_cached = jG;
-        const unsigned long long *curA = sA(sc), *curH = sH(sc);
-        const uint64_t upd = (uint64_t)f[SW_UPD] & SP_KEYMASK, selm = (uint64_t)f[SW_SELM], selb = (uint64_t)f[SW_SELB];
-        const uint64_t clr = ~selm & SP_KEYMASK;
-        const int cap = (int)f[SW_CAP], kb = (int)f[SW_KB], w = (int)f[SW_W];
-        const bool want = f[SW_WANT] != 0;
-        for (uint64_t k = tid; k < n; k += NT) {
-            const unsigned long long x = curA[k];
-            const uint64_t key = x & SP_KEYMASK;
-            const uint32_t v = (uint32_t)(x >> 56);
-            if ((key & selm) == selb) {
-                const uint64_t k2 = key & clr;
-                if ((int)v <= cap && sp_keep(B[b], k2, v)) {
-                    if (sp_insert_min(H, lgn, k2, v) < 0) atomicOr(&c_flag, 1ull);
-                }
-            }
-            if (upd && (int)v < cap) {
-                const uint64_t t = key ^ upd;
-                const uint32_t vc = v + (uint32_t)w;
-                if ((t & selm) == selb) {
-                    const uint64_t t2 = t & clr;
-                    if ((int)vc <= cap && sp_keep(B[b], t2, vc)) {
-                        const uint32_t vo = sp_lookup(curH, lg, t);
-                        const bool hit = vo != 255u;
-                        if (vc < vo && want) {
-                            const unsigned long long q = atomicAdd(&c_ch, 1ull);
-                            if (q < SPW_TINY_N) sCH[q] = t2 | ((unsigned long long)vc << 56);
-                            else atomicOr(&c_flag, 1ull);
-                        }
-                        if (hit || kb < 0 || (int)vc < kb) {
-                            if (sp_insert_min(H, lgn, t2, vc) < 0) atomicOr(&c_flag, 1ull);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        for (uint64_t k = tid; k < capn; k += NT) {
-            const unsigned long long x = H[k];
-            if (x != SP_EMPTY) {
-                const unsigned long long q = atomicAdd(&c_out, 1ull);
-                if (q < SPW_TINY_N) A[q] = x;
-                else atomicOr(&c_flag, 1ull);
-            }
-        }
-        __syncthreads();
-        if (c_flag) { reason = 4; break; }
-        uint64_t nn = c_out;
-        const uint64_t nch = want ? c_ch : 0;
-        const uint64_t jt = (uint64_t)f[SW_JTMASK] & SP_KEYMASK;
-        const unsigned long long *jH = jS ? sJ : jG;
-        unsigned long long best = ~0ull;
-        if (jH)
-            for (uint64_t k = tid; k < nch; k += NT) {
-                const unsigned long long x = sCH[k];
-                const uint32_t bv = sp_lookup(jH, jlg, (x & SP_KEYMASK) ^ jt);
-                if (bv != 255u) best = min(best, (((x >> 56) + bv) << 56) | (x & SP_KEYMASK));
-            }
-        int64_t *o = P.out + 6 * (size_t)i;
-        if (tid == 0) o[5] = (int64_t)nn;
-        int nlg = lgn, ns = os;
-        if (f[SW_TRUNC] >= 0) {
-            if (jH)
-                for (uint64_t k = tid; k < nn; k += NT) {
-                    const unsigned long long x = A[k];
-                    const uint32_t bv = sp_lookup(jH, jlg, (x & SP_KEYMASK) ^ jt);
-                    if (bv != 255u) best = min(best, (((x >> 56) + bv) << 56) | (x & SP_KEYMASK));
-                }
-            int ts = 0;
-            while (ts == os) ts++;
-            const int lgt = lg_for(nn);
-            unsigned long long *T = sH(ts), *TA = sA(ts);
-            for (uint64_t k = tid; k < (1ull << lgt); k += NT) T[k] = SP_EMPTY;
-            __syncthreads();
-            const int below = (int)f[SW_TRUNC];
-            for (uint64_t k = tid; k < nn; k += NT) {
-                const unsigned long long x = A[k];
-                if ((int)(x >> 56) >= below) continue;
-                if (sp_insert_min(T, lgt, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
-                TA[atomicAdd(&c_tr, 1ull)] = x;
-            }
-            __syncthreads();
-            nn = c_tr;
-            nlg = lgt;
-            ns = ts;
-        }
-        if (jH && best != ~0ull) atomicMin(P.res + i, best);
-        int64_t a_off = -1, h_off = -1;
-        if (f[SW_KEEP] == 1 || (f[SW_KEEP] == 2 && nn <= SPW_KEEP_SMALL)) {
-            const int lgk = lg_for(nn);
-            const uint64_t ab = (8 * nn + 255) / 256 * 256, ib = 8ull << lgk;
-            if (used + ab + ib > P.arena_bytes) { reason = 2; break; }
-            unsigned long long *kA = P.arena + used / 8, *kH = P.arena + (used + ab) / 8;
-            const unsigned long long *nA = sA(ns);
-            for (uint64_t k = tid; k < nn; k += NT) kA[k] = nA[k];
-            for (uint64_t k = tid; k < (1ull << lgk); k += NT) kH[k] = SP_EMPTY;
-            __syncthreads();
-            for (uint64_t k = tid; k < nn; k += NT)
-                if (sp_insert_min(kH, lgk, nA[k] & SP_KEYMASK, (uint32_t)(nA[k] >> 56)) < 0) atomicOr(&c_flag, 1ull);
-            a_off = (int64_t)used;
-            h_off = (int64_t)(used + ab);
-            used += ab + ib;
-            if (tid == 0) o[4] = lgk;
-        } else if (tid == 0) {
-            o[4] = nlg;
-        }
-        if (tid == 0) {
-            o[0] = (int64_t)nn;
-            o[1] = (int64_t)nch;
-            o[2] = a_off;
-            o[3] = h_off;
-        }
-        n = nn;
-        lg = nlg;
-        cur = ns;
-        sc = ns;
-        // the next step's rows (fetched above) into the other buffer
-        if (more) {
-            const int nb = b ^ 1;
-            if (tid < SPW_FIELDS) F[nb][tid] = pf;
-            if (tid >= 32 && tid < 32 + (unsigned)SP_MAXCLS && (int)(tid - 32) < P.stride) {
-                B[nb].mask[tid - 32] = pm;
-                B[nb].w[tid - 32] = pw;
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            if (more) {
-                B[b ^ 1].on = (int)F[b ^ 1][SW_USEH];
-                B[b ^ 1].ncls = (int)F[b ^ 1][SW_NCLS];
-                B[b ^ 1].K = P.K;
-                B[b ^ 1].extra = F[b ^ 1][SW_EXTRA];
-                B[b ^ 1].tmask = (uint64_t)F[b ^ 1][SW_TMASK];
-            }
-            c_ch = c_out = c_tr = 0;
-        }
-        __syncthreads();
-    }
-    // the current table back to its global scratch slot (the steps' results are all there)
-    if (i > P.i0 && cur >= 0) {
-        for (uint64_t k = tid; k < n; k += NT) P.arr[cur][k] = sA(sc)[k];
-        for (uint64_t k = tid; k < (1ull << lg); k += NT) P.idx[cur][k] = sH(sc)[k];
-    }
-    if (tid == 0) {
-        P.state[0] = (unsigned long long)i;
-        P.state[1] = (unsigned long long)(long long)cur;
-        P.state[2] = n;
-        P.state[3] = (unsigned long long)lg;
-        P.state[4] = used;
-        P.state[5] = (unsigned long long)reason;
-    }
-}
-
-// stop reasons: 1 a table beyond SPW_SMALL_MAX (continue with the per-step path), 2 arena full,
-// 4 index full, 5 the tables fit the shared-memory walk again
-__global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __grid_constant__ WalkSmall P) {
-    __shared__ unsigned long long c_ch, c_out, c_flag;
-    __shared__ BoundParams B;
-    const unsigned long long *curA = P.A0, *curH = P.H0;
-    uint64_t n = P.n0;
-    int lg = P.lg0, cur = P.slot0;
-    uint64_t used = P.used0;
-    int i = P.i0, reason = 0;
-    const unsigned tid = threadIdx.x, NT = blockDim.x;
-    for (; i < P.nsteps; i++) {
-        const int64_t *f = P.spec + (size_t)SPW_FIELDS * i;
-        if (2 * n > SPW_SMALL_MAX) { reason = 1; break; }
-        if (i > P.i0 && 4 * 2 * n <= SPW_TINY_N && lg <= SPW_TINY_LG) { reason = 5; break; }
-        int os = 0;
-        while (os == cur) os++;
-        const int lgn = lg_for(2 * n);
-        const uint64_t capn = 1ull << lgn;
-        if (tid == 0) {
-            c_ch = c_out = c_flag = 0;
             B.on = (int)f[SW_USEH];
             B.ncls = (int)f[SW_NCLS];
             B.K = P.K;
             B.extra = f[SW_EXTRA];
             B.tmask = (uint64_t)f[SW_TMASK];
         }
-        for (int c = tid; c < (int)f[SW_NCLS] && c < SP_MAXCLS; c += NT) {
-            B.mask[c] = P.masks[(size_t)P.stride * i + c];
-            B.w[c] = P.weights[(size_t)P.stride * i + c];
+        for (int c = tid; c < P.stride && c < SP_MAXCLS; c += NT) {
+            B.mask[c] = P.masks[(size_t)P.stride * step + c];
+            B.w[c] = P.weights[(size_t)P.stride * step + c];
         }
-        unsigned long long *H = P.idx[os];
-        for (uint64_t k = tid; k < capn; k += NT) H[k] = SP_EMPTY;
+    };
+    auto clear = [&](unsigned long long *H, int l) {
+        for (unsigned k = tid; k < (1u << l); k += NT) H[k] = SP_EMPTY;
+    };
+    if (tid < 6) c_cnt[tid / 3][tid % 3] = 0;
+    if (tid == 0) c_flag = 0;
+    const bool go = i < P.nsteps && 2 * n <= limit;
+    if (go) {                                            // the table before step i0, re-indexed
+        load_row(i, i & 1);
+        clear(sH(0), lg);
+        clear(sH(1), lg_tiny(2 * n));
         __syncthreads();
+        for (unsigned k = tid; k < n; k += NT) {
+            const unsigned long long x = P.A0[k];
+            sA(0)[k] = x;
+            if (sp_insert_min(sH(0), lg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+        }
+    }
+    __syncthreads();
+    for (; i < P.nsteps; i++) {
+        if (2 * n > limit) { reason = 1; break; }
+        const int b = i & 1;
+        const int64_t *f = F2[b];
+        const BoundParams &B = B2[b];
+        unsigned long long *cnt = c_cnt[b];
+        const int lgn = lg_tiny(2 * n);
+        const unsigned capn = 1u << lgn;
+        const unsigned long long *curA = sA(sl), *curH = sH(sl);
+        unsigned long long *H = sH(sl ^ 1), *A = sA(sl ^ 1);
+        if (tid < 3) c_cnt[b ^ 1][tid] = 0;              // read last before the barrier that ended step i - 1
         const uint64_t upd = (uint64_t)f[SW_UPD] & SP_KEYMASK, selm = (uint64_t)f[SW_SELM], selb = (uint64_t)f[SW_SELB];
         const uint64_t clr = ~selm & SP_KEYMASK;
         const int cap = (int)f[SW_CAP], kb = (int)f[SW_KB], w = (int)f[SW_W];
         const bool want = f[SW_WANT] != 0;
-        for (uint64_t k = tid; k < n; k += NT) {
-            const unsigned long long x = curA[k];
-            const uint64_t key = x & SP_KEYMASK;
-            const uint32_t v = (uint32_t)(x >> 56);
-            if ((key & selm) == selb) {
-                const uint64_t k2 = key & clr;
-                if ((int)v <= cap && sp_keep(B, k2, v)) {
-                    const int r = sp_insert_min(H, lgn, k2, v);
-                    if (r < 0) atomicOr(&c_flag, 1ull);
+        for (unsigned k0 = 0; k0 < n; k0 += NT) {
+            const unsigned k = k0 + tid;
+            unsigned long long chg = 0;
+            bool changed = false;
+            if (k < n) {
+                const unsigned long long x = curA[k];
+                const uint64_t key = x & SP_KEYMASK;
+                const uint32_t v = (uint32_t)(x >> 56);
+                if ((key & selm) == selb) {
+                    const uint64_t k2 = key & clr;
+                    if ((int)v <= cap && sp_keep(B, k2, v) && sp_insert_min(H, lgn, k2, v) < 0) atomicOr(&c_flag, 1ull);
                 }
-            }
-            if (upd && (int)v < cap) {
-                const uint64_t t = key ^ upd;
-                const uint32_t vc = v + (uint32_t)w;
-                if ((t & selm) == selb) {
+                if (upd && (int)v < cap) {
+                    const uint64_t t = key ^ upd;
+                    const uint32_t vc = v + (uint32_t)w;
                     const uint64_t t2 = t & clr;
-                    if ((int)vc <= cap && sp_keep(B, t2, vc)) {
+                    if ((t & selm) == selb && (int)vc <= cap && sp_keep(B, t2, vc)) {
                         const uint32_t vo = sp_lookup(curH, lg, t);
-                        const bool hit = vo != 255u;
-                        if (vc < vo && want) P.changed[atomicAdd(&c_ch, 1ull)] = t2 | ((unsigned long long)vc << 56);
-                        if (hit || kb < 0 || (int)vc < kb) {
-                            const int r = sp_insert_min(H, lgn, t2, vc);
-                            if (r < 0) atomicOr(&c_flag, 1ull);
-                        }
+                        changed = vc < vo && want;
+                        chg = t2 | ((unsigned long long)vc << 56);
+                        if ((vo != 255u || kb < 0 || (int)vc < kb) && sp_insert_min(H, lgn, t2, vc) < 0)
+                            atomicOr(&c_flag, 1ull);
                     }
                 }
             }
+            if (want) {
+                __syncwarp();
+                const unsigned long long q = sp_claim(&cnt[0], changed);
+                if (changed) sCH[q] = chg;               // at most one a state: n <= SPW_TINY_N / 2
+            }
         }
+        if (i + 1 < P.nsteps) load_row(i + 1, b ^ 1);
         __syncthreads();
-        unsigned long long *A = P.arr[os];
-        for (uint64_t k = tid; k < capn; k += NT) {
+        for (unsigned k = tid; k < capn; k += NT) {      // capn and NT are multiples of the warp
             const unsigned long long x = H[k];
-            if (x != SP_EMPTY) A[atomicAdd(&c_out, 1ull)] = x;
+            const unsigned long long q = sp_claim(&cnt[1], x != SP_EMPTY);
+            if (x != SP_EMPTY) A[q] = x;                 // at most 2 n
         }
         __syncthreads();
         if (c_flag) { reason = 4; break; }
-        uint64_t nn = c_out;
-        const uint64_t nch = want ? c_ch : 0;
-        __syncthreads();                // every thread has read the counters before they are reused
+        uint64_t nn = cnt[1];
+        const uint64_t nch = want ? cnt[0] : 0;
         const unsigned long long *jH = reinterpret_cast<const unsigned long long *>((uintptr_t)f[SW_JTAB]);
         const uint64_t jt = (uint64_t)f[SW_JTMASK] & SP_KEYMASK;
         const int jlg = (int)f[SW_JLG];
         unsigned long long best = ~0ull;
-        if (jH)
-            for (uint64_t k = tid; k < nch; k += NT) {
-                const unsigned long long x = P.changed[k];
+        auto join = [&](const unsigned long long *L, uint64_t m) {
+            for (unsigned k = tid; k < m; k += NT) {
+                const unsigned long long x = L[k];
                 const uint32_t bv = sp_lookup(jH, jlg, (x & SP_KEYMASK) ^ jt);
                 if (bv != 255u) best = min(best, (((x >> 56) + bv) << 56) | (x & SP_KEYMASK));
             }
+        };
+        if (jH) join(sCH, nch);
         int64_t *o = P.out + 6 * (size_t)i;
         if (tid == 0) o[5] = (int64_t)nn;
-        const unsigned long long *nA = A, *nH = H;
-        int nlg = lgn, ns = os;
+        int ns = sl ^ 1, nlg = lgn;
         if (f[SW_TRUNC] >= 0) {
-            if (jH)
-                for (uint64_t k = tid; k < nn; k += NT) {
-                    const unsigned long long x = A[k];
-                    const uint32_t bv = sp_lookup(jH, jlg, (x & SP_KEYMASK) ^ jt);
-                    if (bv != 255u) best = min(best, (((x >> 56) + bv) << 56) | (x & SP_KEYMASK));
-                }
-            int ts = 0;
-            while (ts == os) ts++;
-            const int lgt = lg_for(nn);
-            unsigned long long *T = P.idx[ts], *TA = P.arr[ts];
-            for (uint64_t k = tid; k < (1ull << lgt); k += NT) T[k] = SP_EMPTY;
-            if (tid == 0) c_out = 0;
+            if (jH) join(A, nn);
+            nlg = lg_tiny(nn);
+            unsigned long long *T = sH(sl), *TA = sA(sl);
+            clear(T, nlg);
             __syncthreads();
             const int below = (int)f[SW_TRUNC];
-            for (uint64_t k = tid; k < nn; k += NT) {
-                const unsigned long long x = A[k];
-                if ((int)(x >> 56) >= below) continue;
-                if (sp_insert_min(T, lgt, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
-                TA[atomicAdd(&c_out, 1ull)] = x;
+            for (unsigned k0 = 0; k0 < nn; k0 += NT) {
+                const unsigned k = k0 + tid;
+                const unsigned long long x = k < nn ? A[k] : SP_EMPTY;
+                const bool in = k < nn && (int)(x >> 56) < below;
+                if (in && sp_insert_min(T, nlg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                __syncwarp();
+                const unsigned long long q = sp_claim(&cnt[2], in);
+                if (in) TA[q] = x;
             }
             __syncthreads();
-            nn = c_out;
-            nA = TA;
-            nH = T;
-            nlg = lgt;
-            ns = ts;
+            nn = cnt[2];
+            ns = sl;
         }
-        if (jH && best != ~0ull) atomicMin(P.res + i, best);
+        if (jH) {                                        // one atomic a warp
+            for (int off = 16; off; off >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, off));
+            if ((tid & 31u) == 0 && best != ~0ull) atomicMin(P.res + i, best);
+        }
         int64_t a_off = -1, h_off = -1;
+        unsigned long long *kH = nullptr;                // a smaller index, filled after the barrier
+        int lgk = nlg;
         if (f[SW_KEEP] == 1 || (f[SW_KEEP] == 2 && nn <= SPW_KEEP_SMALL)) {
-            const int lgk = lg_for(nn);
+            const bool copy = nlg <= lg_for(nn) + 1;
+            lgk = copy ? nlg : lg_for(nn);
             const uint64_t ab = (8 * nn + 255) / 256 * 256, ib = 8ull << lgk;
             if (used + ab + ib > P.arena_bytes) { reason = 2; break; }
-            unsigned long long *kA = P.arena + used / 8, *kH = P.arena + (used + ab) / 8;
-            for (uint64_t k = tid; k < nn; k += NT) kA[k] = nA[k];
-            for (uint64_t k = tid; k < (1ull << lgk); k += NT) kH[k] = SP_EMPTY;
-            __syncthreads();
-            for (uint64_t k = tid; k < nn; k += NT)
-                if (sp_insert_min(kH, lgk, kA[k] & SP_KEYMASK, (uint32_t)(kA[k] >> 56)) < 0) atomicOr(&c_flag, 1ull);
+            unsigned long long *kA = P.arena + used / 8, *kI = P.arena + (used + ab) / 8;
+            const unsigned long long *nA = sA(ns), *nH = sH(ns);
+            for (unsigned k = tid; k < nn; k += NT) kA[k] = nA[k];
+            if (copy) {
+                for (unsigned k = tid; k < (1u << lgk); k += NT) kI[k] = nH[k];
+            } else {
+                clear(kI, lgk);
+                kH = kI;
+            }
             a_off = (int64_t)used;
             h_off = (int64_t)(used + ab);
             used += ab + ib;
-            if (tid == 0) o[4] = lgk;   // the working index stays the table's index for the next step
-        } else if (tid == 0) {
-            o[4] = nlg;
         }
         if (tid == 0) {
             o[0] = (int64_t)nn;
             o[1] = (int64_t)nch;
             o[2] = a_off;
             o[3] = h_off;
+            o[4] = lgk;
+        }
+        n = nn;
+        lg = nlg;
+        sl = ns;
+        if (i + 1 < P.nsteps && 2 * n <= limit) clear(sH(sl ^ 1), lg_tiny(2 * n));
+        __syncthreads();
+        if (kH)
+            for (unsigned k = tid; k < n; k += NT) {
+                const unsigned long long x = sA(sl)[k];
+                if (sp_insert_min(kH, lgk, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+            }
+    }
+    // the current table to a global scratch slot (not the one it came from)
+    const int gs = P.slot0 == 0 ? 1 : 0;
+    const bool moved = i > P.i0;
+    if (moved) {
+        for (unsigned k = tid; k < n; k += NT) P.arr[gs][k] = sA(sl)[k];
+        for (unsigned k = tid; k < (1u << lg); k += NT) P.idx[gs][k] = sH(sl)[k];
+    }
+    if (tid == 0) {
+        P.state[0] = (unsigned long long)i;
+        P.state[1] = (unsigned long long)(long long)(moved ? gs : P.slot0);
+        P.state[2] = n;
+        P.state[3] = (unsigned long long)(moved ? lg : P.lg0);
+        P.state[4] = used;
+        P.state[5] = (unsigned long long)reason;
+    }
+}
+
+// The same steps with the tables in the global scratch (L2).  Bound: the chain of dependent accesses of a
+// step between its three barriers (state, old index, new index; claim; kept index), not bytes: the next
+// step's row is fetched during this one, its index is cleared beside the joins and the kept copy, whose
+// index is filled while the next step's states go in; list positions are claimed once per warp.
+// stop reasons: 1 a table beyond the limit (continue with the per-step path), 2 arena full, 4 index
+// full, 5 the tables fit the shared-memory walk again
+__global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __grid_constant__ WalkSmall P) {
+    __shared__ unsigned long long c_cnt[2][3], c_flag;   // per step parity: changed, states, truncated
+    __shared__ BoundParams B2[2];
+    __shared__ int64_t F2[2][SPW_FIELDS];
+    const unsigned long long *curA = P.A0, *curH = P.H0;
+    uint64_t n = P.n0;
+    int lg = P.lg0, cur = P.slot0;
+    uint64_t used = P.used0;
+    int i = P.i0, reason = 0;
+    const unsigned tid = threadIdx.x, NT = blockDim.x;
+    auto load_row = [&](int step, int b) {
+        const int64_t *f = P.spec + (size_t)SPW_FIELDS * step;
+        if (tid < SPW_FIELDS) F2[b][tid] = f[tid];
+        BoundParams &B = B2[b];
+        if (tid == 0) {
+            B.on = (int)f[SW_USEH];
+            B.ncls = (int)f[SW_NCLS];
+            B.K = P.K;
+            B.extra = f[SW_EXTRA];
+            B.tmask = (uint64_t)f[SW_TMASK];
+        }
+        for (int c = tid; c < P.stride && c < SP_MAXCLS; c += NT) {
+            B.mask[c] = P.masks[(size_t)P.stride * step + c];
+            B.w[c] = P.weights[(size_t)P.stride * step + c];
+        }
+    };
+    auto clear = [&](unsigned long long *H, int l) {
+        for (uint64_t k = tid; k < (1ull << l); k += NT) H[k] = SP_EMPTY;
+    };
+    auto out_slot = [](int c) { return c == 0 ? 1 : 0; };
+    if (tid < 6) c_cnt[tid / 3][tid % 3] = 0;
+    if (tid == 0) c_flag = 0;
+    if (i < P.nsteps && 2 * n <= P.limit) {
+        load_row(i, i & 1);
+        clear(P.idx[out_slot(cur)], lg_for(2 * n));
+    }
+    __syncthreads();
+    for (; i < P.nsteps; i++) {
+        if (2 * n > P.limit) { reason = 1; break; }
+        if (i > P.i0 && 2 * 2 * n <= SPW_TINY_N) { reason = 5; break; }
+        const int b = i & 1;
+        const int64_t *f = F2[b];
+        const BoundParams &B = B2[b];
+        unsigned long long *cnt = c_cnt[b];
+        const int os = out_slot(cur), lgn = lg_for(2 * n);
+        const uint64_t capn = 1ull << lgn;
+        unsigned long long *H = P.idx[os], *A = P.arr[os];
+        if (tid < 3) c_cnt[b ^ 1][tid] = 0;              // read last before the barrier that ended step i - 1
+        const uint64_t upd = (uint64_t)f[SW_UPD] & SP_KEYMASK, selm = (uint64_t)f[SW_SELM], selb = (uint64_t)f[SW_SELB];
+        const uint64_t clr = ~selm & SP_KEYMASK;
+        const int cap = (int)f[SW_CAP], kb = (int)f[SW_KB], w = (int)f[SW_W];
+        const bool want = f[SW_WANT] != 0;
+        for (uint64_t k0 = 0; k0 < n; k0 += NT) {
+            const uint64_t k = k0 + tid;
+            unsigned long long chg = 0;
+            bool changed = false;
+            if (k < n) {
+                const unsigned long long x = curA[k];
+                const uint64_t key = x & SP_KEYMASK;
+                const uint32_t v = (uint32_t)(x >> 56);
+                if ((key & selm) == selb) {
+                    const uint64_t k2 = key & clr;
+                    if ((int)v <= cap && sp_keep(B, k2, v) && sp_insert_min(H, lgn, k2, v) < 0) atomicOr(&c_flag, 1ull);
+                }
+                if (upd && (int)v < cap) {
+                    const uint64_t t = key ^ upd;
+                    const uint32_t vc = v + (uint32_t)w;
+                    const uint64_t t2 = t & clr;
+                    if ((t & selm) == selb && (int)vc <= cap && sp_keep(B, t2, vc)) {
+                        const uint32_t vo = sp_lookup(curH, lg, t);
+                        changed = vc < vo && want;
+                        chg = t2 | ((unsigned long long)vc << 56);
+                        if ((vo != 255u || kb < 0 || (int)vc < kb) && sp_insert_min(H, lgn, t2, vc) < 0)
+                            atomicOr(&c_flag, 1ull);
+                    }
+                }
+            }
+            if (want) {
+                __syncwarp();
+                const unsigned long long q = sp_claim(&cnt[0], changed);
+                if (changed) P.changed[q] = chg;
+            }
+        }
+        if (i + 1 < P.nsteps) load_row(i + 1, b ^ 1);
+        __syncthreads();
+        for (uint64_t k = tid; k < capn; k += NT) {      // capn and NT are multiples of the warp
+            const unsigned long long x = H[k];
+            const unsigned long long q = sp_claim(&cnt[1], x != SP_EMPTY);
+            if (x != SP_EMPTY) A[q] = x;
+        }
+        __syncthreads();
+        if (c_flag) { reason = 4; break; }
+        uint64_t nn = cnt[1];
+        const uint64_t nch = want ? cnt[0] : 0;
+        const unsigned long long *jH = reinterpret_cast<const unsigned long long *>((uintptr_t)f[SW_JTAB]);
+        const uint64_t jt = (uint64_t)f[SW_JTMASK] & SP_KEYMASK;
+        const int jlg = (int)f[SW_JLG];
+        unsigned long long best = ~0ull;
+        auto join = [&](const unsigned long long *L, uint64_t m) {
+            for (uint64_t k = tid; k < m; k += NT) {
+                const unsigned long long x = L[k];
+                const uint32_t bv = sp_lookup(jH, jlg, (x & SP_KEYMASK) ^ jt);
+                if (bv != 255u) best = min(best, (((x >> 56) + bv) << 56) | (x & SP_KEYMASK));
+            }
+        };
+        if (jH) join(P.changed, nch);
+        int64_t *o = P.out + 6 * (size_t)i;
+        if (tid == 0) o[5] = (int64_t)nn;
+        const unsigned long long *nA = A, *nH = H;
+        int nlg = lgn, ns = os;
+        if (f[SW_TRUNC] >= 0) {
+            if (jH) join(A, nn);
+            int ts = 0;
+            while (ts == os) ts++;
+            const int lgt = lg_for(nn);
+            unsigned long long *T = P.idx[ts], *TA = P.arr[ts];
+            clear(T, lgt);
+            __syncthreads();
+            const int below = (int)f[SW_TRUNC];
+            for (uint64_t k0 = 0; k0 < nn; k0 += NT) {
+                const uint64_t k = k0 + tid;
+                const unsigned long long x = k < nn ? A[k] : SP_EMPTY;
+                const bool in = k < nn && (int)(x >> 56) < below;
+                if (in && sp_insert_min(T, lgt, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                __syncwarp();
+                const unsigned long long q = sp_claim(&cnt[2], in);
+                if (in) TA[q] = x;
+            }
+            __syncthreads();
+            nn = cnt[2];
+            nA = TA;
+            nH = T;
+            nlg = lgt;
+            ns = ts;
+        }
+        if (jH) {                                        // one atomic a warp
+            for (int off = 16; off; off >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, off));
+            if ((tid & 31u) == 0 && best != ~0ull) atomicMin(P.res + i, best);
+        }
+        int64_t a_off = -1, h_off = -1;
+        unsigned long long *kH = nullptr;
+        int lgk = 0;
+        if (f[SW_KEEP] == 1 || (f[SW_KEEP] == 2 && nn <= SPW_KEEP_SMALL)) {
+            lgk = lg_for(nn);
+            const uint64_t ab = (8 * nn + 255) / 256 * 256, ib = 8ull << lgk;
+            if (used + ab + ib > P.arena_bytes) { reason = 2; break; }
+            unsigned long long *kA = P.arena + used / 8;
+            kH = P.arena + (used + ab) / 8;
+            for (uint64_t k = tid; k < nn; k += NT) kA[k] = nA[k];
+            clear(kH, lgk);
+            a_off = (int64_t)used;
+            h_off = (int64_t)(used + ab);
+            used += ab + ib;
+        }
+        if (tid == 0) {
+            o[0] = (int64_t)nn;
+            o[1] = (int64_t)nch;
+            o[2] = a_off;
+            o[3] = h_off;
+            o[4] = kH ? lgk : nlg;      // the working index stays the table's index for the next step
         }
         curA = nA;
         curH = nH;
         n = nn;
         lg = nlg;
         cur = ns;
+        if (i + 1 < P.nsteps && 2 * n <= P.limit) clear(P.idx[out_slot(cur)], lg_for(2 * n));
         __syncthreads();
+        if (kH)
+            for (uint64_t k = tid; k < n; k += NT)
+                if (sp_insert_min(kH, lgk, curA[k] & SP_KEYMASK, (uint32_t)(curA[k] >> 56)) < 0) atomicOr(&c_flag, 1ull);
     }
     if (tid == 0) {
         P.state[0] = (unsigned long long)i;
@@ -826,7 +887,8 @@ int tg_sp_walk(int nsteps, const int64_t *spec, const uint64_t *masks, const int
     static thread_local size_t dbuf_bytes = 0;
     const size_t b_spec = 8 * (size_t)SPW_FIELDS * nsteps, b_cls = 8 * (size_t)stride * nsteps;
     const size_t b_out = 8 * 6 * (size_t)nsteps, b_all = b_spec + 2 * b_cls + b_out + 64;
-    const bool small_ok = cap_n >= SPW_SMALL_MAX && nsteps > 0;
+    const bool small_ok = cap_n >= SPW_SMALL_MIN && nsteps > 0;
+    const uint64_t limit = std::min<uint64_t>(cap_n, SPW_SMALL_MAX);
     if (small_ok) {
         if (dbuf_bytes < b_all) {
             if (dbuf) cudaFree(dbuf);
@@ -853,8 +915,8 @@ int tg_sp_walk(int nsteps, const int64_t *spec, const uint64_t *masks, const int
     for (int i = 0; i < nsteps; i++) {
         // one-block walks while the tables are small: shared-memory tables first, then global ones;
         // each stops when its tables outgrow it (the small walk also when they become tiny again)
-        while (small_ok && i < nsteps && 2 * n <= SPW_SMALL_MAX) {
-            const bool tiny = 2 * n <= SPW_TINY_N && lg <= SPW_TINY_LG;
+        while (small_ok && i < nsteps && 2 * n <= limit) {
+            const bool tiny = 2 * n <= SPW_TINY_N;
             WalkSmall S;
             S.spec = reinterpret_cast<const int64_t *>(dbuf);
             S.masks = reinterpret_cast<const uint64_t *>(dbuf + b_spec);
@@ -863,6 +925,7 @@ int tg_sp_walk(int nsteps, const int64_t *spec, const uint64_t *masks, const int
             S.K = K;
             S.i0 = i;
             S.nsteps = nsteps;
+            S.limit = limit;
             S.A0 = curA;
             S.H0 = curH;
             S.n0 = n;
@@ -1138,6 +1201,17 @@ int tg_sp_lookup(const void *H, int lg, const void *keys, uint64_t n, void *vals
     if (n) k_sp_lookup<<<sp_grid(n), 256, 0, (cudaStream_t)stream>>>((const unsigned long long *)H, lg,
                                                                      (const unsigned long long *)keys, n, (uint8_t *)vals);
     return cuda_check(cudaGetLastError(), "lookup");
+}
+
+// Traceback through nsteps steps (device rows int64 [nsteps][5]: index of the table before the step
+// (device pointer), its lg, closing bits, column, weight; the last step first) from state s of value v.
+// state: device int64 [3]: the state and value reached, and the steps done (fewer than nsteps where no
+// table holds the path); used: device uint8 [nsteps], 1 where the step used its column.
+int tg_sp_trace(int nsteps, const void *rows, uint64_t s, int v, void *state, void *used, void *stream) {
+    if (nsteps < 0 || (nsteps && (!rows || !used)) || !state) return set_error(TG_ERR_ARG, "bad traceback");
+    k_sp_trace<<<1, 32, 0, (cudaStream_t)stream>>>(static_cast<const int64_t *>(rows), nsteps, s, v,
+                                                   static_cast<uint8_t *>(used), static_cast<int64_t *>(state));
+    return cuda_check(cudaGetLastError(), "traceback");
 }
 
 // Value histogram of an array into hist (device, 256 x uint64, zeroed by the call).

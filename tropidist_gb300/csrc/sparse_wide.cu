@@ -94,7 +94,7 @@ __device__ __forceinline__ bool spw_keep(const WideBound &b, const uint64_t (&k)
         for (int w = 0; w < W; w++) cnt += __popcll((k[w] ^ b.tmask[w]) & b.mask[c][w]);
         tot += b.w[c] * (int64_t)cnt;
     }
-    return (int64_t)v + (tot + SPW_QW - 1) / SPW_QW <= (int64_t)b.K;
+    return tot <= ((int64_t)b.K - (int64_t)v) * SPW_QW;     // v + ceil(tot / QW) <= K
 }
 
 // value of key in a table's index (255 when absent)
@@ -401,6 +401,49 @@ __global__ void k_spw_lookup(const unsigned long long *__restrict__ H, int lg, c
     }
 }
 
+// The traceback through a run of steps on W-word states (k_sp_trace of sparse.cu): rows int64
+// [5 + 2 W]: index, lg, keys, key stride, weight, closing bits, column; state: [0 .. W - 1] the state,
+// [W] its value, [W + 1] steps done.
+template <int W>
+__global__ void k_spw_trace(const int64_t *__restrict__ rows, int n, uint64_t *state, uint8_t *used) {
+    const unsigned lane = threadIdx.x;
+    uint64_t s[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) s[w] = state[w];
+    int v = (int)state[W], i = 0;
+    for (; i < n; i++) {
+        const int64_t *r = rows + (size_t)(5 + 2 * W) * i;
+        uint64_t k[W];
+        bool any = false;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            const uint64_t col = (uint64_t)r[5 + W + w];
+            any = any || col != 0;
+            s[w] |= (uint64_t)r[5 + w];
+            k[w] = lane ? s[w] ^ col : s[w];
+        }
+        uint32_t val = 255u;
+        if (lane < 2)
+            val = spw_lookup<W>(reinterpret_cast<const unsigned long long *>((uintptr_t)r[0]), (int)r[1],
+                                reinterpret_cast<const uint64_t *>((uintptr_t)r[2]), (uint64_t)r[3], k);
+        const int without = (int)__shfl_sync(0xffffffffu, val, 0), with_col = (int)__shfl_sync(0xffffffffu, val, 1);
+        const bool take = without != v;
+        if (take && (!any || with_col != v - (int)r[4])) break;
+        if (take) {
+#pragma unroll
+            for (int w = 0; w < W; w++) s[w] ^= (uint64_t)r[5 + W + w];
+            v -= (int)r[4];
+        }
+        if (lane == 0) used[i] = take ? 1 : 0;
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int w = 0; w < W; w++) state[w] = s[w];
+        state[W] = (uint64_t)v;
+        state[W + 1] = (uint64_t)i;
+    }
+}
+
 // ---- kernels of a walk: the table sizes and index widths stay on the device between steps
 #define SPW_TAG (1ull << 39)          // join result from a whole table (not the changed list)
 #define SPW_KEEP_SMALL 1024           // keep mode 2: only tables of at most this many states
@@ -443,8 +486,8 @@ __global__ void k_spw_keep_alloc(const unsigned long long *n_dev, uint64_t ncap,
 }
 
 __device__ __forceinline__ unsigned long long *spw_keep_index(uint8_t *arena, const unsigned long long *rec, int W) {
-    const uint64_t stride = rec[4];
-    return reinterpret_cast<unsigned long long *>(arena + rec[1] + (uint64_t)W * stride * 8 + (stride + 255) / 256 * 256);
+    const uint64_t stride = __ldcg(rec + 4);
+    return reinterpret_cast<unsigned long long *>(arena + __ldcg(rec + 1) + (uint64_t)W * stride * 8 + (stride + 255) / 256 * 256);
 }
 
 __global__ void k_spw_keep_fill(uint8_t *arena, const unsigned long long *rec, int W) {
@@ -456,10 +499,10 @@ template <int W>
 __device__ __forceinline__ void spw_keep_body(const Lanes &L, const uint64_t *__restrict__ keys,
                                               const uint8_t *__restrict__ vals, uint64_t n, uint64_t stride,
                                               uint8_t *arena, unsigned long long *rec) {
-    const uint64_t ks = rec[4];
-    uint64_t *nk = reinterpret_cast<uint64_t *>(arena + rec[1]);
-    uint8_t *nv = arena + rec[1] + (uint64_t)W * ks * 8;
-    spw_filter_body<W>(L, keys, vals, n, stride, -1, nk, nv, ks, spw_keep_index(arena, rec, W), (int)rec[3], rec);
+    const uint64_t ks = __ldcg(rec + 4), off = __ldcg(rec + 1);
+    uint64_t *nk = reinterpret_cast<uint64_t *>(arena + off);
+    uint8_t *nv = arena + off + (uint64_t)W * ks * 8;
+    spw_filter_body<W>(L, keys, vals, n, stride, -1, nk, nv, ks, spw_keep_index(arena, rec, W), (int)__ldcg(rec + 3), rec);
 }
 
 template <int W>
@@ -474,7 +517,7 @@ template <int W>
 __device__ __forceinline__ void spw_capture_one(const unsigned long long *result, const uint64_t *ck,
                                                 const uint8_t *cv, const uint64_t *tk, const uint8_t *tv,
                                                 uint64_t stride, uint64_t *resk, uint8_t *resv) {
-    const unsigned long long r = *result;
+    const unsigned long long r = __ldcg(result);
     if (r == SPW_EMPTY) return;
     const uint64_t i = r & (SPW_TAG - 1);
     const uint64_t *k = (r & SPW_TAG) ? tk : ck;
@@ -539,8 +582,9 @@ __host__ __device__ __forceinline__ int spw_prev_off(const int64_t *steps, int i
     return 8 * i;
 }
 
-#define SPW_SMALL_THREADS 512
-static uint64_t g_spw_small_limit = 512;       // the one-block walk steps tables while 2 n <= this
+#define SPW_SMALL_THREADS 1024
+#define SPW_SMALL_DEFAULT 4096
+static uint64_t g_spw_small_limit = SPW_SMALL_DEFAULT;   // the one-block walk steps tables while 2 n <= this
 
 struct SpwSmall {
     const int64_t *steps;             // device copies of the walk's step records
@@ -554,33 +598,32 @@ struct SpwSmall {
     uint8_t *resv, *arena;
 };
 
-// Steps i0.. of a walk in one block while the tables are small (no launch per kernel of a step):
-// the same bodies as the separate kernels, with the block's barriers between them.  Stops before a
-// step whose table holds more than limit / 2 states (reason 1) or after a step that raised a flag
-// (reason 4, the walk is void); state: [0] next step, [1] ring slot of its table, [2] reason.
+// Steps i0.. of a walk in one block while the tables are small (no launch per kernel of a step): the
+// same bodies as the separate kernels, with the block's barriers between them.  Stops before a step
+// whose table holds more than limit / 2 states (reason 1) or after a step that raised a flag (reason 4,
+// the walk is void); state: [0] next step, [1] ring slot of its table, [2] reason.
+//
+// Bound: the chain of dependent L2 accesses of a step (row, state, index probe, claim), not bytes.
+// The next step's row is fetched during this one, its indexes are cleared beside this step's kept copy,
+// and that copy is written while the next step's states go in.  Three-word states, host included: 20 to
+// 27 us a step at 300 to 1000 states, where the separate launches take 55 to 65 (host-bound); 17 us at
+// 10 states, before 25.
 template <int W>
 __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_spw_walk_small(const __grid_constant__ SpwSmall S) {
-    __shared__ WideStep P;
-    __shared__ WideBound B;
-    __shared__ uint64_t jt[SPW_MAXW];
+    __shared__ WideStep P2[2];
+    __shared__ WideBound B2[2];
+    __shared__ uint64_t jt2[2][SPW_MAXW];
     const Lanes L = block_lanes();
     const unsigned tid = threadIdx.x;
+    const bool lead = tid == 0;
     unsigned long long *abort = S.cnt + 8ull * (2 * (uint64_t)S.nsteps + 1) + 1, *state = abort + 1;
     const uint64_t cap = S.cap;
-    int cur = S.cur, i = S.i0, reason = 0;
-    for (; i < S.nsteps; i++) {
-        int noff, lgoff;
-        const unsigned long long *pc = S.cnt + spw_prev_off(S.steps, i, noff, lgoff);
-        const uint64_t n = spw_count(pc + noff, cap);
-        const int lg_old = (int)__ldcg(pc + lgoff);
-        if (__ldcg(abort)) { reason = 4; break; }
-        if (2 * n > S.limit) { reason = 1; break; }
+    auto load_row = [&](int i, int b) {                  // this block's copy of step i's parameters
         const int64_t *f = S.steps + (size_t)SPW_WALK_FIELDS * i;
         const uint64_t *wd = S.words + (size_t)5 * W * i;
-        const unsigned long long *jH = reinterpret_cast<const unsigned long long *>((uintptr_t)f[WK_JH]);
-        const uint64_t *jk = reinterpret_cast<const uint64_t *>((uintptr_t)f[WK_JKEYS]);
-        const bool join = f[WK_JOIN] && jH && jk;
         const int ncls = f[WK_USEH] ? (int)f[WK_NCLS] : 0;
+        WideStep &P = P2[b];
+        WideBound &B = B2[b];
         if (tid == 0) {
             P.cap = (int)f[WK_CAP];
             P.keep_below = (int)f[WK_KB];
@@ -596,20 +639,44 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_spw_walk_small(const __gr
             P.sel_mask[q] = wd[W + q];
             P.sel_bits[q] = wd[2 * W + q];
             B.tmask[q] = wd[3 * W + q];
-            jt[q] = wd[4 * W + q];
+            jt2[b][q] = wd[4 * W + q];
         }
         for (unsigned c = tid; c < (unsigned)(ncls * W); c += blockDim.x)
             B.mask[c / W][c % W] = S.masks[((size_t)i * S.maxc) * W + c];
         for (unsigned c = tid; c < (unsigned)ncls; c += blockDim.x) B.w[c] = S.weights[(size_t)i * S.maxc + c];
-        unsigned long long *c = S.cnt + 8ull * (i + 1);
+    };
+    int cur = S.cur, i = S.i0, reason = 0;
+    uint64_t n = 0;
+    int lg_old = 0;
+    {
+        int noff, lgoff;
+        const unsigned long long *pc = S.cnt + spw_prev_off(S.steps, i, noff, lgoff);
+        n = spw_count(pc + noff, cap);
+        lg_old = (int)__ldcg(pc + lgoff);
+    }
+    if (i < S.nsteps && 2 * n <= S.limit) {
+        load_row(i, i & 1);
         const int lgs = spw_lg_dev(2 * n);
-        if (tid == 0) c[3] = (unsigned long long)lgs;
-        const int out = (cur + 1) % 3;
         spw_fill_body(L, S.sg.H, 1ull << lgs);
-        spw_fill_body(L, S.ring[out].H, 1ull << lgs);
-        __syncthreads();
-        spw_emit_body<W, true>(L, S.ring[cur].keys, S.ring[cur].vals, n, cap, S.sg.keys, S.sg.vals, 2 * cap, S.sg.H, lgs,
-                               P, B, c);
+        spw_fill_body(L, S.ring[(cur + 1) % 3].H, 1ull << lgs);
+    }
+    if (__ldcg(abort)) reason = 4;
+    __syncthreads();
+    for (; i < S.nsteps && !reason; i++) {
+        if (2 * n > S.limit) { reason = 1; break; }
+        const WideStep &P = P2[i & 1];
+        const WideBound &B = B2[i & 1];
+        const int64_t *f = S.steps + (size_t)SPW_WALK_FIELDS * i;
+        const unsigned long long *jH = reinterpret_cast<const unsigned long long *>((uintptr_t)f[WK_JH]);
+        const uint64_t *jk = reinterpret_cast<const uint64_t *>((uintptr_t)f[WK_JKEYS]);
+        const bool join = f[WK_JOIN] && jH && jk;
+        unsigned long long *c = S.cnt + 8ull * (i + 1), *rec = S.cnt + 8ull * (S.nsteps + 1 + i);
+        const int lgs = spw_lg_dev(2 * n);
+        if (lead) c[3] = (unsigned long long)lgs;
+        const int out = (cur + 1) % 3;
+        spw_emit_body<W, true>(L, S.ring[cur].keys, S.ring[cur].vals, n, cap, S.sg.keys, S.sg.vals, 2 * cap, S.sg.H, lgs, P, B,
+                         c);
+        if (i + 1 < S.nsteps) load_row(i + 1, (i + 1) & 1);
         __syncthreads();
         spw_compact_body<W>(L, S.sg.H, 1ull << lgs, S.sg.keys, 2 * cap, S.ring[out].keys, S.ring[out].vals, cap,
                             S.ring[out].H, lgs, S.ch.keys, S.ch.vals, cap, S.ring[cur].H, lg_old, S.ring[cur].keys,
@@ -619,44 +686,45 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_spw_walk_small(const __gr
         const uint64_t nout = spw_count(c, cap);
         if (join)
             spw_join_body<W>(L, S.ch.keys, S.ch.vals, spw_count(c + 1, cap), cap, jH, (int)f[WK_JLG], jk,
-                             (uint64_t)f[WK_JSTRIDE], jt, S.res + i, 0);
-        int now = out;
-        const unsigned long long *nnow = c;
+                             (uint64_t)f[WK_JSTRIDE], jt2[i & 1], S.res + i, 0);
+        int now = out, lgn = lgs;
+        uint64_t nnow = nout;
         if (f[WK_TRUNC] >= 0) {
             // the cap drops at this cut: the whole table before the drop is joined too
             if (join)
                 spw_join_body<W>(L, S.ring[out].keys, S.ring[out].vals, nout, cap, jH, (int)f[WK_JLG], jk,
-                                 (uint64_t)f[WK_JSTRIDE], jt, S.res + i, SPW_TAG);
-            const int tr = (out + 1) % 3, lgt = spw_lg_dev(nout);
-            if (tid == 0) c[5] = (unsigned long long)lgt;
-            spw_fill_body(L, S.ring[tr].H, 1ull << lgt);
+                                 (uint64_t)f[WK_JSTRIDE], jt2[i & 1], S.res + i, SPW_TAG);
+            now = (out + 1) % 3;
+            lgn = spw_lg_dev(nout);
+            if (lead) c[5] = (unsigned long long)lgn;
+            spw_fill_body(L, S.ring[now].H, 1ull << lgn);
             __syncthreads();
-            spw_filter_body<W>(L, S.ring[out].keys, S.ring[out].vals, nout, cap, (int)f[WK_TRUNC], S.ring[tr].keys,
-                               S.ring[tr].vals, cap, S.ring[tr].H, lgt, c + 4);
-            now = tr;
-            nnow = c + 4;
+            spw_filter_body<W>(L, S.ring[out].keys, S.ring[out].vals, nout, cap, (int)f[WK_TRUNC], S.ring[now].keys,
+                               S.ring[now].vals, cap, S.ring[now].H, lgn, c + 4);
+            __syncthreads();
+            if (__ldcg(c + 6) & 7ull) { reason = 4; break; }
+            nnow = spw_count(c + 4, cap);
         }
+        if (f[WK_KEEP] && lead) spw_keep_place(nnow, W, (int)f[WK_KEEP], rec, abort - 1, S.arena ? S.arena_bytes : 0);
         __syncthreads();
-        if (__ldcg(c + 6) & 7ull) { reason = 4; break; }
-        if (join && tid == 0)
+        const bool keep = f[WK_KEEP] && !(__ldcg(rec + 2) & 24ull);
+        if (join && lead)
             spw_capture_one<W>(S.res + i, S.ch.keys, S.ch.vals, S.ring[out].keys, S.ring[out].vals, cap,
                                S.resk + (size_t)i * W, S.resv + i);
-        if (f[WK_KEEP]) {
-            unsigned long long *rec = S.cnt + 8ull * (S.nsteps + 1 + i);
-            const uint64_t nk = spw_count(nnow, cap);
-            if (tid == 0) spw_keep_place(nk, W, (int)f[WK_KEEP], rec, abort - 1, S.arena ? S.arena_bytes : 0);
-            __syncthreads();
-            if (!(__ldcg(rec + 2) & 24ull)) {
-                spw_fill_body(L, spw_keep_index(S.arena, rec, W), 1ull << __ldcg(rec + 3));
-                __syncthreads();
-                spw_keep_body<W>(L, S.ring[now].keys, S.ring[now].vals, nk, cap, S.arena, rec);
-            }
+        if (keep) spw_fill_body(L, spw_keep_index(S.arena, rec, W), 1ull << __ldcg(rec + 3));
+        cur = now;
+        n = nnow;
+        lg_old = lgn;
+        if (i + 1 < S.nsteps && 2 * n <= S.limit) {      // the next step's staging and new index
+            const int lgx = spw_lg_dev(2 * n);
+            spw_fill_body(L, S.sg.H, 1ull << lgx);
+            spw_fill_body(L, S.ring[(cur + 1) % 3].H, 1ull << lgx);
         }
         __syncthreads();
-        cur = now;
+        if (keep) spw_keep_body<W>(L, S.ring[cur].keys, S.ring[cur].vals, n, cap, S.arena, rec);
     }
-    if (reason == 4 && tid == 0) *abort = 1;
-    if (tid == 0) {
+    if (lead) {
+        if (reason == 4) *abort = 1;
         state[0] = (unsigned long long)i;
         state[1] = (unsigned long long)cur;
         state[2] = (unsigned long long)reason;
@@ -831,7 +899,13 @@ static int spw_walk_w(int nsteps, const int64_t *steps, const uint64_t *words, c
     if (n0)
         k_spw_filter<W><<<spw_grid(n0), 256, 0, st>>>(k0, v0, n0, stride0, -1, ring[0].keys, ring[0].vals, cap,
                                                       ring[0].H, 0, cnt, nullptr, cnt + 3);
-    const uint64_t limit = std::min<uint64_t>(g_spw_small_limit, cap);
+    // tables of 1 to 4096 states (n <= limit / 2): one block a step; a walk that holds a step with values
+    // beyond 8 bits leaves it to the separate launches, which refuse it, from 256 states up
+    uint64_t limit = std::min<uint64_t>(g_spw_small_limit, cap);
+    for (int q = 0; q < nsteps; q++) {
+        const int64_t *f = steps + (size_t)SPW_WALK_FIELDS * q;
+        if (f[WK_CAP] > 254 || f[WK_W] < 1 || f[WK_W] > 254) limit = std::min<uint64_t>(limit, 512);
+    }
     uint64_t host_n = n0;             // the table size before step i, when known on the host
     int cur = 0, i = 0;
     while (i < nsteps) {
@@ -977,6 +1051,21 @@ using namespace tg;
     }
 
 extern "C" {
+
+// Traceback on multi-word states (as tg_sp_trace): rows device int64 [nsteps][5 + 2 W], state device
+// uint64 [W + 2] in and out (the state, its value, steps done), used device uint8 [nsteps].
+int tg_spw_trace(int W, int nsteps, const void *rows, void *state, void *used, void *stream) {
+    int e = spw_check_words(W);
+    if (e) return e;
+    if (nsteps < 0 || (nsteps && (!rows || !used)) || !state) return set_error(TG_ERR_ARG, "bad traceback");
+#define SPW_TRACE(WW)                                                                                              \
+    (k_spw_trace<WW><<<1, 32, 0, (cudaStream_t)stream>>>(static_cast<const int64_t *>(rows), nsteps,               \
+                                                        static_cast<uint64_t *>(state),                            \
+                                                        static_cast<uint8_t *>(used)),                             \
+     cuda_check(cudaGetLastError(), "traceback"))
+    SPW_DISPATCH(W, SPW_TRACE);
+#undef SPW_TRACE
+}
 
 int tg_spw_step(int W, const void *keys, const void *vals, uint64_t n, uint64_t stride, const void *Hold, int lg_old,
                 void *ekeys, void *evals, uint64_t ecap, void *Hs, int lgs, void *nkeys, void *nvals, uint64_t ncap,

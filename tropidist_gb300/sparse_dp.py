@@ -635,7 +635,7 @@ class Sweep:
                     continue
                 t, tmask = j
                 steps[k, 5] = 1
-                steps[k, 9], steps[k, 10] = t.keys.data_ptr(), t.H.data_ptr()
+                steps[k, 9], steps[k, 10] = t.kptr(), t.hptr()
                 steps[k, 11], steps[k, 12] = t.lg, t.stride
                 words[k, 4] = words_of(tmask, W)
         return steps, words, masks0[pos], weights0[pos]
@@ -726,6 +726,13 @@ class Sweep:
                 tabs = self.tables(c + 1, hi)
                 steps = [(p, tabs[p + 1]) for p in range(c, hi)]
                 c = hi
+            if self.legs:                # device tables: the whole interval in one call
+                ps = [p for p, _ in steps]
+                flags, s, v, done = self.be.trace([t for _, t in steps], [tr.col[p] for p in ps], [sel[p] for p in ps],
+                                                  [tr.cw[p] for p in ps], s, v)
+                assert done == len(ps), "traceback lost the path"
+                used.extend(tr.order[p] for p, u in zip(ps, flags.tolist()) if u)
+                continue
             for p, before in steps:
                 mid = s | sel[p]
                 without, with_col = _values(self.be, before, [mid, mid ^ tr.col[p]])

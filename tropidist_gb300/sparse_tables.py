@@ -274,6 +274,25 @@ class GpuTables:
         self._arena_guess = max(1 << 16, used + (used >> 2))
         return out[:m], kept, (res[:m].cpu().numpy().view(U64) if want_res else None)
 
+    def trace(self, tabs, cols, sels, weights, s, v):
+        """Traceback through the tables `tabs` (each the table before its step, the last step first)
+        from state s of value v: (used flags uint8 [m], state, value, steps done); csrc/sparse.cu
+        tg_sp_trace."""
+        m = len(tabs)
+        rows = np.empty((max(1, m), 5), dtype=np.int64)
+        if m:
+            rows[:, 0] = [t.hptr() for t in tabs]
+            rows[:, 1] = [t.lg for t in tabs]
+            rows[:, 2] = np.array(sels, dtype=U64).view(np.int64)
+            rows[:, 3] = np.array(cols, dtype=U64).view(np.int64)
+            rows[:, 4] = weights
+        dev = self.torch.from_numpy(rows).cuda()
+        out = self._empty(3 + (m + 7) // 8)          # state, value, steps done, then the flags
+        _lib.check(self.L.tg_sp_trace(m, dev.data_ptr(), int(s), int(v), out.data_ptr(), out.data_ptr() + 24,
+                                      device.stream_ptr()))
+        o = out.cpu().numpy()
+        return o[3:].view(np.uint8)[:m], int(o[0]), int(o[1]), int(o[2])
+
     def hist(self, tab):
         import torch
         h = torch.zeros(256, dtype=torch.int64, device="cuda")
@@ -322,6 +341,50 @@ class _WTab:
 
     def __init__(self, keys, vals, n, stride, H, lg):
         self.keys, self.vals, self.n, self.stride, self.H, self.lg = keys, vals, n, stride, H, lg
+
+    def kptr(self):
+        return self.keys.data_ptr()
+
+    def hptr(self):
+        return self.H.data_ptr()
+
+
+class _WArenaTab:
+    """A wide table kept by a device walk inside the walk's arena (byte offset o: keys, values, index);
+    the tensor views are made only when asked for."""
+    __slots__ = ("arena", "o", "n", "stride", "lg", "W")
+
+    def __init__(self, arena, o, n, stride, lg, W):
+        self.arena, self.o, self.n, self.stride, self.lg, self.W = arena, o, n, stride, lg, W
+
+    def _vo(self):
+        return self.o + 8 * self.W * self.stride
+
+    def _ho(self):
+        return self._vo() + (self.stride + 255) // 256 * 256
+
+    def kptr(self):
+        return self.arena.data_ptr() + self.o
+
+    def hptr(self):
+        return self.arena.data_ptr() + self._ho()
+
+    @property
+    def keys(self):
+        return self.arena[self.o // 8:self.o // 8 + self.W * self.stride]
+
+    @property
+    def vals(self):
+        return self.arena.view(dtype=_torch_u8())[self._vo():self._vo() + self.stride]
+
+    @property
+    def H(self):
+        return self.arena[self._ho() // 8:self._ho() // 8 + (1 << self.lg)]
+
+
+def _torch_u8():
+    import torch
+    return torch.uint8
 
 
 class WideGpuTables:
@@ -518,16 +581,36 @@ class WideGpuTables:
                 arena_bytes = max(arena_bytes + (arena_bytes >> 1), int(need[1]) + (1 << 20))
         self._walk_cap = cap
         kept, used = {}, 0
-        u8 = arena.view(torch.uint8)
-        for i in np.nonzero(out[:m, 2] >= 0)[0].tolist():
-            n, o, st, lg = (int(x) for x in out[i, [0, 2, 3, 4]])
-            vo = o + 8 * W * st
-            ho = vo + (st + 255) // 256 * 256
-            kept[i] = _WTab(arena[o // 8:o // 8 + W * st], u8[vo:vo + st], n, st, arena[ho // 8:ho // 8 + (1 << lg)],
-                            lg)
-            used = max(used, ho + (8 << lg))
+        ks = np.nonzero(out[:m, 2] >= 0)[0]
+        for i, (n, o, st, lg) in zip(ks.tolist(), out[ks][:, [0, 2, 3, 4]].tolist()):
+            t = kept[i] = _WArenaTab(arena, o, n, st, lg, W)
+            used = max(used, t._ho() + (8 << lg))
         self._arena_guess = max(1 << 16, used + (used >> 2))
         return out[:m], kept, (res[:m] if want_res else None)
+
+    def trace(self, tabs, cols, sels, weights, s, v):
+        """As GpuTables.trace on states of W words (csrc/sparse_wide.cu tg_spw_trace)."""
+        m, W = len(tabs), self.W
+        rows = np.empty((max(1, m), 5 + 2 * W), dtype=np.int64)
+        if m:
+            rows[:, 0] = [t.hptr() for t in tabs]
+            rows[:, 1] = [t.lg for t in tabs]
+            rows[:, 2] = [t.kptr() for t in tabs]
+            rows[:, 3] = [t.stride for t in tabs]
+            rows[:, 4] = weights
+            for w in range(W):
+                rows[:, 5 + w] = np.array([(int(x) >> (64 * w)) & M64 for x in sels], dtype=U64).view(np.int64)
+                rows[:, 5 + W + w] = np.array([(int(x) >> (64 * w)) & M64 for x in cols], dtype=U64).view(np.int64)
+        # the rows, then the state, value, steps done and flags
+        host = np.zeros(rows.size + W + 2 + (m + 7) // 8, dtype=np.int64)
+        host[:rows.size] = rows.reshape(-1)
+        host[rows.size:rows.size + W] = self._w(s).view(np.int64)
+        host[rows.size + W] = int(v)
+        dev = self.torch.from_numpy(host).cuda()
+        at = dev.data_ptr() + 8 * rows.size
+        _lib.check(self.L.tg_spw_trace(W, m, dev.data_ptr(), at, at + 8 * (W + 2), device.stream_ptr()))
+        o = dev[rows.size:].cpu().numpy()
+        return o[W + 2:].view(np.uint8)[:m], ints_of(o[None, :W].view(U64))[0], int(o[W]), int(o[W + 1])
 
     @staticmethod
     def walk_best(res):
