@@ -48,9 +48,10 @@ def _plans(p, order):
     """One plan per logical observable; the span form of H is shared (cdist/auto.py:67-76)."""
     hrows = trellis.minimal_span_form(trellis.rows_from_columns(p.h, order, p.nrows))
     pw = None if getattr(p, "weights", None) is None else [p.weights[j] for j in order]
-    for i in range(p.nobs):
-        lrow = trellis.reduce_target_row(trellis.target_row(p.l, 1 << i, order), hrows)
-        yield i, trellis.make_plan(hrows, lrow, len(order), pw)
+    by_ends, hbytes = trellis.span_ends(hrows), trellis.row_bytes(hrows, len(order))
+    for i, target in enumerate(trellis.target_rows(p.l, p.nobs, order)):
+        lrow = trellis.reduce_target_row(target, hrows, by_ends)
+        yield i, trellis.make_plan(hrows, lrow, len(order), pw, hbytes)
 
 
 def estimate(p, order=None, max_table_bytes=None):

@@ -18,11 +18,16 @@
 #include "dense_types.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <functional>
+#include <string>
+#include <thread>
 #include <vector>
 
 namespace tg {
+
+extern thread_local std::string g_err;
 
 #define BJ_NONE 0xFFFFFFFFu
 #define BJ_UNIT_CHUNKS 4096u
@@ -260,6 +265,72 @@ static const void *fill_job(const Seg &S, BJob &J, size_t &bytes) {
     return S.kind == 4 ? (const void *)&S.gp : (const void *)&S.pp;
 }
 
+// One plan of a batch, scheduled: its jobs in order (offsets within its own parameter blob), or why not.
+struct PlanJobs {
+    int status = TG_OK;
+    std::string error;
+    int peak_bits = 0, final_buf = 0;
+    std::vector<BJob> jobs;
+    std::vector<uint8_t> params;
+};
+
+static void schedule_plan(const int64_t *ops, int64_t nops, PlanJobs &Q) {
+    try {
+        if (nops < 0) {
+            Q.status = TG_ERR_ARG;
+            Q.error = "bad plan offsets";
+            return;
+        }
+        DensePlan P;
+        Q.status = build_dense_plan(ops, nops, 1, nullptr, 0, P);
+        if (Q.status) {
+            Q.error = g_err;
+            return;
+        }
+        for (const Seg &S : P.segs) {
+            if ((S.kind == 0 && S.sp.max_bits > 15) || (S.kind == 1 && S.pp.d > 16)) {
+                Q.status = TG_ERR_TOO_BIG;
+                Q.error = "batched plans need sweeps of <= 15 bits and tiles of <= 16 bits";
+                return;
+            }
+            BJob J;
+            memset(&J, 0, sizeof(J));
+            size_t bytes;
+            const void *rec = fill_job(S, J, bytes);
+            if (bytes) {
+                J.params_off = align_up(Q.params.size(), 16);
+                Q.params.resize(J.params_off + bytes);
+                memcpy(Q.params.data() + J.params_off, rec, bytes);
+            }
+            Q.jobs.push_back(J);
+        }
+        Q.peak_bits = P.peak_bits;
+        Q.final_buf = P.final_buf;
+    } catch (const std::exception &) {
+        Q.status = TG_ERR_NOMEM;
+        Q.error = "out of host memory while scheduling a plan";
+    }
+}
+
+// Every plan of a batch, on up to 16 host threads (a plan takes 0.3 to 4 ms to schedule and plans are
+// independent); the calling thread takes part, so a thread that cannot be started costs only time.
+static void schedule_plans(int nplans, const int64_t *ops, const int64_t *offsets, std::vector<PlanJobs> &out) {
+    sm_count();                        // looked up once, before the threads read it
+    std::atomic<int> next(0);
+    auto work = [&]() {
+        for (int i; (i = next.fetch_add(1)) < nplans;)
+            schedule_plan(ops + 3 * offsets[i], offsets[i + 1] - offsets[i], out[i]);
+    };
+    const int want = std::min<int>({16, (int)std::max(1u, std::thread::hardware_concurrency()), nplans / 4}) - 1;
+    std::vector<std::thread> pool;
+    try {
+        for (int t = 0; t < want; t++) pool.emplace_back(work);
+    } catch (const std::exception &) {
+    }
+    work();
+    for (std::thread &t : pool) t.join();
+}
+
 static_assert(sizeof(BJob) % 16 == 0, "job descriptors are read as 16-byte words");
 
 static bool g_batch_attr = false;
@@ -471,47 +542,42 @@ void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, in
         B->first.assign(nplans, BJ_NONE);
         B->final_off.assign(nplans, 0);
         B->width.assign(nplans, 0);
+        std::vector<PlanJobs> pj(nplans);
+        schedule_plans(nplans, ops, offsets, pj);
+        size_t njobs = 0, nprm = 0;
+        for (const PlanJobs &Q : pj) {
+            njobs += Q.jobs.size();
+            nprm += align_up(Q.params.size(), 16);
+        }
+        B->jobs.reserve(njobs);
+        B->params.reserve(nprm);
         for (int i = 0; i < nplans && !st; i++) {
-            const int64_t n = offsets[i + 1] - offsets[i];
-            if (n < 0) { st = set_error(TG_ERR_ARG, "bad plan offsets"); break; }
-            DensePlan P;
-            st = build_dense_plan(ops + 3 * offsets[i], n, 1, nullptr, 0, P);
-            if (st) break;
-            for (const Seg &S : P.segs)
-                if ((S.kind == 0 && S.sp.max_bits > 15) || (S.kind == 1 && S.pp.d > 16)) {
-                    st = set_error(TG_ERR_TOO_BIG, "batched plans need sweeps of <= 15 bits and tiles of <= 16 bits");
-                    break;
-                }
-            if (st) break;
-            B->width[i] = P.peak_bits;
-            const uint64_t tb = align_up((size_t)1 << P.peak_bits, 256);
+            PlanJobs &Q = pj[i];
+            if (Q.status) {
+                st = set_error(Q.status, Q.error.c_str());
+                break;
+            }
+            B->width[i] = Q.peak_bits;
+            const uint64_t tb = align_up((size_t)1 << Q.peak_bits, 256);
             const uint64_t a = B->arena_bytes, b = a + tb;
             B->arena_bytes = b + tb;
-            B->final_off[i] = P.final_buf ? b : a;
-            int cur = 0;
-            unsigned prev = BJ_NONE;
-            for (const Seg &S : P.segs) {
-                BJob J;
-                memset(&J, 0, sizeof(J));
+            B->final_off[i] = Q.final_buf ? b : a;
+            const unsigned base = (unsigned)B->jobs.size();
+            if (!Q.jobs.empty()) B->first[i] = base;
+            const size_t poff = align_up(B->params.size(), 16);
+            B->params.resize(poff);
+            B->params.insert(B->params.end(), Q.params.begin(), Q.params.end());
+            for (size_t k = 0; k < Q.jobs.size(); k++) {
+                BJob J = Q.jobs[k];
                 J.plan = i;
-                J.next = BJ_NONE;
-                J.src_off = cur ? b : a;
-                J.dst_off = cur ? a : b;
-                size_t bytes;
-                const void *rec = fill_job(S, J, bytes);
-                if (bytes) {
-                    J.params_off = align_up(B->params.size(), 16);
-                    B->params.resize(J.params_off + bytes);
-                    memcpy(B->params.data() + J.params_off, rec, bytes);
-                }
+                J.next = k + 1 < Q.jobs.size() ? base + (unsigned)k + 1 : BJ_NONE;
+                J.src_off = k & 1 ? b : a;
+                J.dst_off = k & 1 ? a : b;
+                J.params_off += poff;
                 B->units += J.nunits;
-                const unsigned idx = (unsigned)B->jobs.size();
-                if (prev == BJ_NONE) B->first[i] = idx;
-                else B->jobs[prev].next = idx;
                 B->jobs.push_back(J);
-                prev = idx;
-                cur ^= 1;
             }
+            Q = PlanJobs();
         }
         if (!st) {
             const size_t nj = std::max<size_t>(1, B->jobs.size());

@@ -236,10 +236,13 @@ struct Seg {
     uint32_t op_b = 0;
     int w_in, w_out;
     int64_t op_end;         // ops done after this segment
-    SweepParams sp;
-    PassParams pp;
-    GranParams gp;
     int ckpt = -1;          // index of a checkpoint written after this segment
+    union {                 // the kind's parameters (a plan holds hundreds of segments of several KB)
+        SweepParams sp;
+        PassParams pp;
+        GranParams gp;
+    };
+    Seg() {}
 };
 
 struct DensePlan {

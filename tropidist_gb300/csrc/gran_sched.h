@@ -160,46 +160,58 @@ static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, in
     for (int m = 0; m < nc; m++)
         if (cols[m].type == GC_N || cols[m].type == GC_C) loaded[nl++] = m;
     if (nl + nsw != L) return -2;
-    bool busy[GP_SLOTS];
     int lims[GP_MAXOPS];
-    // assigns the opening columns' slots, fills lims; returns the members gone through, -1 if it does not fit
-    auto assign = [&]() {
+    uint32_t live_slots = 0;
+    // assigns the opening columns' slots and fills lims; returns the members gone through, or -1 once
+    // they reach `bound`
+    auto assign = [&](int bound) {
         int work = 0;
-        for (int s = 0; s < GP_SLOTS; s++) busy[s] = s < L;
-        for (int m = 0; m < nc; m++) {
-            GranCol &C = cols[m];
-            if (C.type == GC_O) {
-                int s = 0;
-                while (s < GP_SLOTS && busy[s]) s++;
-                if (s == GP_SLOTS) return -1;
-                C.slot = s;
+        uint32_t m = (1u << L) - 1u;                     // live slots
+        for (int c = 0; c < nc; c++) {
+            GranCol &C = cols[c];
+            if (C.type == GC_O) C.slot = __builtin_ctz(~m);
+            int n;                                       // the highest live slot decides
+            if (C.type == GC_I1) {
+                n = 32;
+                work += n;
+            } else if (C.type == GC_A) {
+                n = m >= 16 ? 32 : m >= 8 ? 16 : 8;
+                work += n;
+            } else {
+                const uint32_t lo = m & ((1u << C.slot) - 1u), o = lo | ((m >> (C.slot + 1)) << C.slot);
+                n = o >= 8 ? 16 : o >= 4 ? 8 : 4;
+                work += 2 * n;
             }
-            int n = C.type == GC_I1 || C.type == GC_A ? 32 : 16;
-            for (int s = GP_SLOTS - 1; s >= 0 && C.type != GC_I1; s--) {
-                if (s == C.slot) continue;
-                if (busy[s] || n <= (C.type == GC_A ? 8 : 4)) break;
-                n >>= 1;
-            }
-            lims[m] = n;
-            work += C.type == GC_A || C.type == GC_I1 ? n : 2 * n;
-            if (C.type == GC_O) busy[C.slot] = true;
-            if (C.type == GC_C) busy[C.slot] = false;
+            lims[c] = n;
+            if (work >= bound) return -1;
+            if (C.type == GC_O) m |= 1u << C.slot;
+            if (C.type == GC_C) m &= ~(1u << C.slot);
         }
+        live_slots = m;
         return work;
     };
-    int perm[GP_SLOTS], best_perm[GP_SLOTS], best_work = INT32_MAX;
+    // orders of the loaded columns (the N columns among themselves keep theirs), from the one that puts the
+    // first to close highest
+    int perm[GP_SLOTS], best_perm[GP_SLOTS], best_work = INT32_MAX, nn = 0;
+    for (int q = 0; q < nl; q++) nn += cols[loaded[q]].type == GC_N;
+    std::stable_partition(loaded, loaded + nl, [&](int m) { return cols[m].type == GC_N; });
+    std::reverse(loaded + nn, loaded + nl);
     for (int q = 0; q < nl; q++) perm[q] = q;
     do {
+        bool skip = false;
+        for (int q = 0; q + 1 < nn; q++) skip |= perm[q] > perm[q + 1];
+        if (skip) continue;
         for (int q = 0; q < nl; q++) cols[loaded[q]].slot = nsw + perm[q];
-        const int w = assign();
-        if (w >= 0 && w < best_work) {
-            best_work = w;
-            std::copy(perm, perm + nl, best_perm);
-        }
+        const int w = assign(best_work);
+        if (w < 0) continue;
+        best_work = w;
+        std::copy(perm, perm + nl, best_perm);
     } while (std::next_permutation(perm, perm + nl));
     if (best_work == INT32_MAX) return -2;
     for (int q = 0; q < nl; q++) cols[loaded[q]].slot = nsw + best_perm[q];
-    assign();
+    assign(INT32_MAX);
+    bool busy[GP_SLOTS];
+    for (int s = 0; s < GP_SLOTS; s++) busy[s] = (live_slots >> s) & 1u;
     // ---- coset-number bits: the input rows that are neither pivots nor fixed, by position
     uint64_t piv = 0;
     for (int q = 0; q < nb; q++) piv |= 1ull << top(basis[q]);

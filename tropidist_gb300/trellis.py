@@ -103,6 +103,12 @@ def cut_profile(cols, order):
     return [a + b - tot for a, b in zip(fwd, bwd)]
 
 
+def row_bytes(rows, ncols):
+    """Rows (bitmasks over ncols positions) as whole little-endian 64-bit words."""
+    nb = 8 * max(1, (ncols + 63) // 64)
+    return b"".join(r.to_bytes(nb, "little") for r in rows)
+
+
 def rows_from_columns(cols, order, nrows):
     """Row r as a bitmask over column positions of `order`."""
     rows = [0] * nrows
@@ -155,11 +161,15 @@ def minimal_span_form(rows):
     return out
 
 
-def reduce_target_row(lrow, hrows):
+def span_ends(hrows):
+    """The constraint rows by first and by last position, for reducing several target rows."""
+    return {lowbit(r): r for r in hrows}, {r.bit_length(): r for r in hrows}
+
+
+def reduce_target_row(lrow, hrows, by_ends=None):
     """Shorten the span of the target-1 row with the constraint rows; 0 means the query is
-    infeasible (the observable is a combination of the checks)."""
-    starts = {lowbit(r): r for r in hrows}
-    ends = {r.bit_length(): r for r in hrows}
+    infeasible (the observable is a combination of the checks).  by_ends: span_ends(hrows)."""
+    starts, ends = span_ends(hrows) if by_ends is None else by_ends
 
     def strip_start(x):
         while x:
@@ -256,28 +266,28 @@ def encode_ops(ops):
     return out
 
 
-def make_plan(hrows, lrow, ncols, weights=None):
+def make_plan(hrows, lrow, ncols, weights=None, hbytes=None):
     """Op stream of the sweep for constraint rows (target 0) and one target-1 row
     (cdist/trellis.py:147-182), built by the library's C++ planner (tg_make_plan) from the rows as
-    bitsets.  weights: optional per-position column weight."""
+    bitsets.  weights: optional per-position column weight.  hbytes: row_bytes(hrows, ncols), for
+    callers that plan several target rows over the same constraint rows."""
     if lrow == 0:
         return Plan([], 0, [], ncols, feasible=False)
     import ctypes
     from . import _lib
-    rows = list(hrows) + [lrow]
+    nrows = len(hrows) + 1
     words = max(1, (ncols + 63) // 64)
-    nb = 8 * words
-    buf = b"".join(r.to_bytes(nb, "little") for r in rows)
+    buf = (row_bytes(hrows, ncols) if hbytes is None else hbytes) + row_bytes([lrow], ncols)
     bits = np.frombuffer(buf, dtype=np.uint64)
     w = None if weights is None else np.ascontiguousarray(weights, dtype=np.int64)
     widths = np.zeros(max(1, ncols), dtype=np.int32)
     out = np.zeros(3, dtype=np.int64)
-    cap = 2 * len(rows) + ncols + 16
+    cap = 2 * nrows + ncols + 16
     L = _lib.lib()
     while True:
         ops = np.zeros((cap, 3), dtype=np.int64)
         cols = np.zeros(cap, dtype=np.int32)
-        r = L.tg_make_plan(len(rows), ncols, words, bits.ctypes.data, w.ctypes.data if w is not None else None,
+        r = L.tg_make_plan(nrows, ncols, words, bits.ctypes.data, w.ctypes.data if w is not None else None,
                            ops.ctypes.data, cap, widths.ctypes.data, cols.ctypes.data, out.ctypes.data)
         if r == -4:
             raise ValueError("update masks are limited to 63 bits")
@@ -331,6 +341,16 @@ def target_row(l, obs_mask, order):
         if bin(l[j] & obs_mask).count("1") & 1:
             lrow |= 1 << pos
     return lrow
+
+
+def target_rows(l, nobs, order):
+    """target_row of every single observable: [target_row(l, 1 << i, order) for i in range(nobs)]."""
+    if nobs > 63 or not order or max(l) >> 63:
+        return [target_row(l, 1 << i, order) for i in range(nobs)]
+    bits = np.array([l[j] for j in order], dtype=np.int64)
+    one = np.int64(1)
+    return [int.from_bytes(np.packbits(((bits >> np.int64(i)) & one).astype(np.uint8), bitorder="little").tobytes(),
+                           "little") for i in range(nobs)]
 
 
 def build_plan(h, l, obs_mask, order, nrows, weights=None):
