@@ -1695,6 +1695,166 @@ __global__ void __launch_bounds__(1024) k_witness_small(const int64_t *ops, int6
     out[2 + out_cap] = status;
 }
 
+// ---- the same with the table in shared memory (tables of at most 2^WS_TABLE_BITS bytes, WS_MAXOPS ops).
+// Ops are applied in place there, and only the tables before updates are kept in `tabs`, each at a
+// 16-byte boundary: an op costs a few barriers instead of a round trip through L2.  The walk back reads the table before an update at the current state and at its
+// partner; one warp reads five updates ahead, a lane for every outcome of the ones between, so that five
+// updates cost one memory latency.
+#define WS_TABLE_BITS 17
+#define WS_MAXOPS 4096
+#define WS_THREADS 1024
+#define WS_AHEAD 5
+
+__host__ __device__ __forceinline__ uint64_t ws_room(int w, size_t eb) { return ((eb << w) + 15) / 16 * 16; }
+
+// ops: (mask | position, code | (weight | target) << 2)
+template <typename E>
+__global__ void __launch_bounds__(WS_THREADS) k_witness_smem(const uint2 *__restrict__ ops, int n, uint8_t *tabs,
+                                                             int32_t *out, int64_t out_cap) {
+    constexpr uint32_t INF = Entry<E>::INF;
+    constexpr int CB = Entry<E>::CB;
+    extern __shared__ uint4 smem_raw[];
+    E *T = reinterpret_cast<E *>(smem_raw);
+    __shared__ uint2 s_ops[WS_MAXOPS];
+    const unsigned tid = threadIdx.x, NT = blockDim.x;
+    for (unsigned k = tid; k < (unsigned)n; k += NT) s_ops[k] = ops[k];
+    if (tid == 0) T[0] = 0;
+    __syncthreads();
+    uint64_t off = 0;
+    int w = 0;
+    for (int k = 0; k < n; k++) {
+        const uint2 op = s_ops[k];
+        const uint32_t code = op.y & 3u, arg = op.y >> 2;
+        const uint32_t m = 1u << w;
+        if (code == 0) {
+            if (w >= CB) {
+                for (uint32_t c = tid; c < (m >> CB); c += NT) smem_raw[(m >> CB) + c] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            } else if (tid < m) {
+                T[m + tid] = (E)INF;
+            }
+            w++;
+        } else if (code == 1) {
+            if (w >= CB) {
+                uint4 *D = reinterpret_cast<uint4 *>(tabs + off);
+                for (uint32_t c = tid; c < (m >> CB); c += NT) D[c] = smem_raw[c];
+            } else if (tid < m) {
+                reinterpret_cast<E *>(tabs + off)[tid] = T[tid];
+            }
+            off += ws_room(w, sizeof(E));
+            __syncthreads();
+            smem_update<E>(T, w, op.x, arg);
+        } else {
+            const int pos = (int)op.x;
+            const uint32_t half = m >> 1;
+            if (w - 1 >= CB) {           // at most 2^(WS_TABLE_BITS - 1) bytes out: 4 chunks a thread
+                uint4 v[(1 << (WS_TABLE_BITS - 5)) / WS_THREADS];
+                const uint32_t nch = half >> CB;
+#pragma unroll
+                for (int q = 0; q < (1 << (WS_TABLE_BITS - 5)) / WS_THREADS; q++) {
+                    const uint32_t c = q * NT + tid;
+                    if (c >= nch) continue;
+                    if (pos >= CB) {
+                        v[q] = smem_raw[insert_zero(c, pos - CB) | (arg << (pos - CB))];
+                    } else {
+                        E *e = reinterpret_cast<E *>(&v[q]);
+#pragma unroll
+                        for (uint32_t j = 0; j < (1u << CB); j++)
+                            e[j] = T[insert_zero((c << CB) | j, pos) | (arg << pos)];
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < (1 << (WS_TABLE_BITS - 5)) / WS_THREADS; q++) {
+                    const uint32_t c = q * NT + tid;
+                    if (c < nch) smem_raw[c] = v[q];
+                }
+            } else {
+                const E v = tid < half ? T[insert_zero(tid, pos) | (arg << pos)] : (E)0;
+                __syncthreads();
+                if (tid < half) T[tid] = v;
+            }
+            w--;
+        }
+        __syncthreads();
+    }
+    if (tid >= 32) return;
+    const uint32_t value = T[0];
+    int64_t used = 0;
+    int status = 0;
+    if (w == 0 && value != INF) {
+        const int lane = (int)tid, level = 31 - __clz(lane + 1), prefix = lane + 1 - (1 << level);
+        uint32_t st = 0, v = value;
+        int k = n - 1;
+        while (k >= 0 && !status) {
+            // this lane: the update `level` updates back, had the ones before it gone as `prefix` says
+            uint32_t x = st, here = ~0u, partner = ~0u;
+            {
+                uint64_t o = off;
+                int ww = w, lev = 0;
+                for (int q = k; q >= 0 && level < WS_AHEAD; q--) {
+                    const uint2 op = s_ops[q];
+                    const uint32_t code = op.y & 3u;
+                    if (code == 2) {
+                        x = insert_zero(x, (int)op.x) | ((op.y >> 2) << op.x);
+                        ww++;
+                    } else if (code == 0) {
+                        ww--;
+                    } else {
+                        o -= ws_room(ww, sizeof(E));
+                        if (lev == level) {
+                            if (!(x >> ww)) {
+                                const E *B = reinterpret_cast<const E *>(tabs + o);
+                                here = __ldcg(B + x);
+                                partner = __ldcg(B + (x ^ op.x));
+                            }
+                            break;
+                        }
+                        if ((prefix >> lev) & 1) x ^= op.x;
+                        lev++;
+                    }
+                }
+            }
+            // the real outcomes, one update after the other
+            int lev = 0, path = 0;
+            for (; k >= 0 && lev < WS_AHEAD && !status; k--) {
+                const uint2 op = s_ops[k];
+                const uint32_t code = op.y & 3u;
+                if (code == 2) {
+                    st = insert_zero(st, (int)op.x) | ((op.y >> 2) << op.x);
+                    w++;
+                } else if (code == 0) {
+                    w--;
+                    if (st >> w) status = 2;
+                } else {
+                    off -= ws_room(w, sizeof(E));
+                    const int src = (1 << lev) - 1 + path;
+                    const uint32_t h = __shfl_sync(0xffffffffu, here, src), p = __shfl_sync(0xffffffffu, partner, src);
+                    if (h != v) {
+                        st ^= op.x;
+                        v -= op.y >> 2;
+                        if (p != v) {
+                            status = 2;
+                        } else {
+                            if (lane == 0 && used < out_cap) out[2 + used] = (int32_t)k;
+                            used++;
+                        }
+                        path |= 1 << lev;
+                    }
+                    lev++;
+                }
+            }
+        }
+        if (!status && (st != 0 || v != 0)) status = 2;
+    } else if (w != 0) {
+        status = 1;
+    }
+    if (tid == 0) {
+        out[0] = (int32_t)value;
+        out[1] = (int32_t)used;
+        out[2 + out_cap] = status;
+    }
+}
+
 }  // namespace tg
 
 using namespace tg;
@@ -2030,6 +2190,33 @@ int tg_dense_witness_small(const int64_t *ops, int64_t n, int eb, void *tables, 
     if (need < 0) return set_error(TG_ERR_ARG, "bad op stream");
     if ((uint64_t)need > table_bytes) return set_error(TG_ERR_TOO_BIG, "witness tables larger than the buffer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // tables of at most 2^WS_TABLE_BITS bytes and a stream without errors: shared memory (240 columns at 15
+    // bits, the whole call: 1.38 ms through L2, 0.77 ms here); anything else takes the tables through L2
+    std::vector<uint2> packed;
+    size_t peak = 16;
+    if (n <= WS_MAXOPS && ((uintptr_t)tables & 15) == 0) {
+        int w = 0;
+        uint64_t room = 0;
+        bool fits = true;
+        for (int64_t k = 0; k < n && fits; k++) {
+            const int64_t code = ops[3 * k], a = ops[3 * k + 1], b = ops[3 * k + 2];
+            if (code == 0) {
+                w++;
+                peak = std::max(peak, (size_t)eb << w);
+                fits = ((size_t)eb << w) <= (1u << WS_TABLE_BITS);
+                packed.push_back(make_uint2(0, 0));
+            } else if (code == 1) {
+                fits = a > 0 && !((uint64_t)a >> w) && b >= 1 && b <= (eb == 1 ? 254 : 65534);
+                room += ws_room(w, eb);
+                packed.push_back(make_uint2((uint32_t)a, 1u | ((uint32_t)b << 2)));
+            } else {
+                fits = code == 2 && a >= 0 && a < w && (b == 0 || b == 1);
+                w--;
+                packed.push_back(make_uint2((uint32_t)a, 2u | ((uint32_t)b << 2)));
+            }
+        }
+        if (!fits || room > table_bytes) packed.clear();
+    }
     static thread_local int64_t *dops = nullptr;
     static thread_local int64_t dops_n = 0;
     if (dops_n < n) {
@@ -2042,9 +2229,22 @@ int tg_dense_witness_small(const int64_t *ops, int64_t n, int eb, void *tables, 
         }
         dops_n = n;
     }
-    int e = TG_OK;
+    int e = cuda_check(cudaMemsetAsync(out_dev, 0, 4 * (size_t)(3 + out_cap), st), "witness out");
+    if (!e && !packed.empty()) {
+        e = cuda_check(cudaMemcpyAsync(dops, packed.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, st), "witness ops");
+        const void *fn = eb == 1 ? (const void *)k_witness_smem<uint8_t> : (const void *)k_witness_smem<uint16_t>;
+        if (!e) e = cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 1 << WS_TABLE_BITS),
+                               "witness shared memory");
+        if (e) return e;
+        if (eb == 1)
+            k_witness_smem<uint8_t><<<1, WS_THREADS, peak, st>>>(reinterpret_cast<const uint2 *>(dops), (int)n,
+                                                                 static_cast<uint8_t *>(tables), out_dev, out_cap);
+        else
+            k_witness_smem<uint16_t><<<1, WS_THREADS, peak, st>>>(reinterpret_cast<const uint2 *>(dops), (int)n,
+                                                                  static_cast<uint8_t *>(tables), out_dev, out_cap);
+        return cuda_check(cudaGetLastError(), "witness kernel");
+    }
     if (n) e = cuda_check(cudaMemcpyAsync(dops, ops, 24 * (size_t)n, cudaMemcpyHostToDevice, st), "witness ops");
-    if (!e) e = cuda_check(cudaMemsetAsync(out_dev, 0, 4 * (size_t)(3 + out_cap), st), "witness out");
     if (e) return e;
     const uint64_t cap = (uint64_t)need / eb;
     if (eb == 1)
