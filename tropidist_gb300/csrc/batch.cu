@@ -117,8 +117,61 @@ __host__ __device__ __forceinline__ uint64_t gran_steps(const GranParams &P) {
     return (P.ncosets + FP_THREADS - 1) >> FP_TBITS;
 }
 
-// one unit of a job by the whole block: TC = three 64 KB tile buffers, PRM = parameter copy
-__device__ void run_unit(const BJob &J, unsigned unit, uint8_t *arena, const uint8_t *params, uint4 *TC, uint4 *PRM) {
+#define BT_TILE_SMEM (3 * 65536)
+// The tiles [t0, t1) of a fused pass in its plainest form: load, INF over the opened rows, updates in
+// shared memory, store.  For relayout passes (no updates), and in the granule kernels for any other
+// pass that a plan holds.
+static __device__ __forceinline__ void plain_tiles(const PassParams &P, uint64_t t0, uint64_t t1, const uint8_t *in,
+                                                   uint8_t *out, uint4 *TC) {
+    constexpr int CB = 4;
+    const int nb_in = P.d_in - CB, nb_out = P.d_out - CB;
+    const uint32_t nch_in = 1u << nb_in, nch_all = 1u << (P.d - CB), nch_out = 1u << nb_out;
+    for (uint64_t t = t0; t < t1; t++) {
+        uint64_t ib = 0, ob = 0;
+        for (int k = 0; k < P.n_outer; k++)
+            if ((t >> k) & 1ull) { ib += P.outer_in[k]; ob += P.outer_out[k]; }
+        for (uint32_t c = threadIdx.x; c < nch_in; c += BT_THREADS)
+            cp_async16(TC + c, in + ib + pdep_w64(c, P.loc_in + CB, nb_in));
+        for (uint32_t c = nch_in + threadIdx.x; c < nch_all; c += BT_THREADS) TC[c] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        cp_async_wait_all();
+        __syncthreads();
+        for (int u = 0; u < P.nupd; u++) {
+            smem_update<uint8_t>(reinterpret_cast<uint8_t *>(TC), P.d, P.upd_mask[u], P.upd_w[u]);
+            __syncthreads();
+        }
+        for (uint32_t q = threadIdx.x; q < nch_out; q += BT_THREADS) {
+            const uint64_t off = ob + pdep_w64(q, P.cmp_out + CB, nb_out);
+            const uint32_t sidx = pdep_w32(q, P.cmp_smem + CB, nb_out) + P.sel_bits;
+            *reinterpret_cast<uint4 *>(out + off) = u8_out_chunk(TC, P.fast_out ? 0 : 2, sidx, P, 0u);
+        }
+        __syncthreads();
+    }
+}
+
+// a tile or chunk-streaming pass in its fast form: TC = three 64 KB tile buffers
+static __device__ __noinline__ void fast_pass(const BJob &J, unsigned unit, const uint8_t *src, uint8_t *dst, uint4 *TC,
+                                              uint4 *PRM) {
+    const PassParams &P = *reinterpret_cast<const PassParams *>(PRM);
+    const uint64_t t0 = (uint64_t)unit * J.grain;
+    const uint64_t nt = P.stream ? (P.ntiles + (1ull << (9 - P.nkt)) - 1) >> (9 - P.nkt) : P.ntiles;
+    const uint64_t t1 = t0 + J.grain < nt ? t0 + J.grain : nt;
+    if (P.stream) u8_stream_range(P, t0, t1, src, dst, TC);     // a unit: a range of steps
+    else if (P.use_groups) u8_pass_range(P, t0, t1, src, dst, TC);
+    else
+        for (uint64_t t = t0; t < t1; t++) {
+            u8_tile<BT_THREADS>(P, t, src, dst, TC);
+            __syncthreads();
+        }
+}
+
+// One unit of a job by the whole block; PRM = the block's copy of the job's parameters.  FAST: the passes
+// other than granule passes run in their fast forms.  A kernel that holds those (their register arrays,
+// a call) spills 4 KB a thread in the granule step, so the kernels come in both kinds and the one without
+// is used unless more than one pass in eight is of another form (a plan under the default knobs has a
+// stray one where two rows open or close at one column).
+template <bool FAST>
+static __device__ __forceinline__ void run_unit(const BJob &J, unsigned unit, uint8_t *arena, const uint8_t *params,
+                                                uint4 *TC, uint4 *PRM) {
     const uint8_t *src = arena + J.src_off;
     uint8_t *dst = arena + J.dst_off;
     if (J.kind != 2) {
@@ -126,28 +179,27 @@ __device__ void run_unit(const BJob &J, unsigned unit, uint8_t *arena, const uin
         const uint4 *g = reinterpret_cast<const uint4 *>(params + J.params_off);
         for (uint32_t i = threadIdx.x; i < (psize + 15) / 16; i += blockDim.x) PRM[i] = __ldcg(g + i);
         __syncthreads();
-        if (J.kind == 0) {
-            sweep_body<uint8_t>(*reinterpret_cast<const SweepParams *>(PRM), src, dst, TC);
-        } else if (J.kind == 3) {
-            const GranParams &P = *reinterpret_cast<const GranParams *>(PRM);
-            const uint32_t n = (uint32_t)gran_steps(P), s0 = unit * J.grain, s1 = min(s0 + J.grain, n);
-            for (uint32_t s = s0; s < s1; s++)
-                gran_step<1, FP_TBITS, false>(P, s, reinterpret_cast<const uint32_t *>(src), reinterpret_cast<uint32_t *>(dst));
-        } else {
-            const PassParams &P = *reinterpret_cast<const PassParams *>(PRM);
-            const uint64_t t0 = (uint64_t)unit * J.grain;
-            const uint64_t nt = P.stream ? (P.ntiles + (1ull << (9 - P.nkt)) - 1) >> (9 - P.nkt) : P.ntiles;
-            const uint64_t t1 = t0 + J.grain < nt ? t0 + J.grain : nt;
-            if (P.stream) u8_stream_range(P, t0, t1, src, dst, TC);     // a unit: a range of steps
-            else if (P.use_groups) u8_pass_range(P, t0, t1, src, dst, TC);
-            else
-                for (uint64_t t = t0; t < t1; t++) {
-                    u8_tile<BT_THREADS>(P, t, src, dst, TC);
-                    __syncthreads();
-                }
+    }
+    if (J.kind == 3) {
+        const GranParams &P = *reinterpret_cast<const GranParams *>(PRM);
+        const uint32_t n = (uint32_t)gran_steps(P), s0 = unit * J.grain, s1 = min(s0 + J.grain, n);
+        for (uint32_t s = s0; s < s1; s++) {
+            asm volatile("" ::: "memory");       // the parameters are read again at every step: kept they spill
+            gran_step<1, FP_TBITS, false>(P, s, reinterpret_cast<const uint32_t *>(src), reinterpret_cast<uint32_t *>(dst));
         }
     } else {
-        batch_single_op(J, unit, src, dst);
+        if (J.kind == 0) {
+            sweep_body<uint8_t>(*reinterpret_cast<const SweepParams *>(PRM), src, dst, TC);
+        } else if (J.kind == 1 && FAST) {
+            fast_pass(J, unit, src, dst, TC, PRM);
+        } else if (J.kind == 1) {
+            const PassParams &P = *reinterpret_cast<const PassParams *>(PRM);
+            const int g = P.stream ? 9 - P.nkt : 0;      // log2 of the tiles per counted item
+            const uint64_t t0 = ((uint64_t)unit * J.grain) << g, t1 = t0 + ((uint64_t)J.grain << g);
+            plain_tiles(P, t0, t1 < P.ntiles ? t1 : P.ntiles, src, dst, TC);
+        } else {
+            batch_single_op(J, unit, src, dst);
+        }
     }
 }
 
@@ -161,14 +213,14 @@ __device__ __forceinline__ BJob load_job(const BJob *p) {
     return J;
 }
 
-#define BT_TILE_SMEM (3 * 65536)
-__global__ void __launch_bounds__(BT_THREADS, 1) k_batch(const __grid_constant__ BatchArgs A) {
+template <bool FAST> __global__ void __launch_bounds__(BT_THREADS, 1) k_batch(const __grid_constant__ BatchArgs A) {
     extern __shared__ uint4 smem_raw[];
     // layout: three 64 KB tile buffers (a sweep uses the first two), then the job's parameters
     uint4 *TC = smem_raw;
     uint4 *PRM = smem_raw + (BT_TILE_SMEM / 16);
     __shared__ int s_state;
     __shared__ unsigned s_job, s_unit;
+    __shared__ BJob s_J;                 // in shared memory: the granule step needs the registers
     for (;;) {
         if (threadIdx.x == 0) {
             int st;
@@ -177,11 +229,12 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_batch(const __grid_constant__
             s_state = st;
             s_job = j;
             s_unit = u;
+            if (st == 0) s_J = A.jobs[j];
         }
         __syncthreads();
         if (s_state != 0) break;
-        const BJob J = A.jobs[s_job];
-        run_unit(J, s_unit, A.arena, A.params, TC, PRM);
+        const BJob &J = s_J;
+        run_unit<FAST>(J, s_unit, A.arena, A.params, TC, PRM);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -218,6 +271,7 @@ struct BatchPlan {
     std::vector<uint64_t> final_off;     // arena offset of each plan's final table
     std::vector<int> width;              // peak width of each plan
     uint64_t arena_bytes = 0;
+    int64_t ngran = 0, nother = 0;       // granule passes, other passes with updates
     int64_t units = 0;
     void *dev = nullptr;                 // jobs, params, counters
     size_t dev_bytes = 0;
@@ -270,6 +324,7 @@ struct PlanJobs {
     int status = TG_OK;
     std::string error;
     int peak_bits = 0, final_buf = 0;
+    int64_t ngran = 0, nother = 0;
     std::vector<BJob> jobs;
     std::vector<uint8_t> params;
 };
@@ -293,6 +348,8 @@ static void schedule_plan(const int64_t *ops, int64_t nops, PlanJobs &Q) {
                 Q.error = "batched plans need sweeps of <= 15 bits and tiles of <= 16 bits";
                 return;
             }
+            Q.ngran += S.kind == 4;
+            Q.nother += S.kind == 1 && S.pp.nupd > 0;
             BJob J;
             memset(&J, 0, sizeof(J));
             size_t bytes;
@@ -393,7 +450,7 @@ __device__ void server_grab(const ServerArgs &A, int &state, unsigned &job, unsi
     state = 1;
 }
 
-__global__ void __launch_bounds__(BT_THREADS, 1) k_server(const __grid_constant__ ServerArgs A) {
+template <bool FAST> __global__ void __launch_bounds__(BT_THREADS, 1) k_server(const __grid_constant__ ServerArgs A) {
     extern __shared__ uint4 smem_raw[];
     uint4 *TC = smem_raw;
     uint4 *PRM = smem_raw + (BT_TILE_SMEM / 16);
@@ -413,8 +470,8 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_server(const __grid_constant_
         }
         __syncthreads();
         if (s_state != 0) break;
-        const BJob J = s_J;
-        run_unit(J, s_unit, A.arena, A.params, TC, PRM);
+        const BJob &J = s_J;
+        run_unit<FAST>(J, s_unit, A.arena, A.params, TC, PRM);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -491,6 +548,9 @@ struct Server {
     std::vector<unsigned> free_slots;    // kept sorted, highest first: low slots are reused first
     unsigned mbox_tail = 0;
     int blocks = 0;
+    bool fast = false;                   // a plan with many passes of the other forms was admitted: launches from
+                                         // then on take the kernel that holds them (one that runs already
+                                         // takes such passes in their plain form)
     bool launched = false;
     unsigned *h_buf = nullptr;           // pinned: plan_done flags, then the control words
 };
@@ -514,11 +574,14 @@ static int server_launch(Server &S) {
     A.idle_limit = 20000ull;        // about 5-10 ms of polling without work, then the blocks leave
     static bool attr = false;
     if (!attr) {
-        const int e = cuda_check(cudaFuncSetAttribute(k_server, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
+        int e = cuda_check(cudaFuncSetAttribute(k_server<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
+        if (!e)
+            e = cuda_check(cudaFuncSetAttribute(k_server<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
         if (e) return e;
         attr = true;
     }
-    k_server<<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
+    if (S.fast) k_server<true><<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
+    else k_server<false><<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
     S.launched = true;
     return cuda_check(cudaGetLastError(), "server launch");
 }
@@ -558,6 +621,8 @@ void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, in
                 break;
             }
             B->width[i] = Q.peak_bits;
+            B->ngran += Q.ngran;
+            B->nother += Q.nother;
             const uint64_t tb = align_up((size_t)1 << Q.peak_bits, 256);
             const uint64_t a = B->arena_bytes, b = a + tb;
             B->arena_bytes = b + tb;
@@ -682,7 +747,9 @@ int tg_batch_run(void *p, void *arena, int blocks, int window, uint32_t *values,
         if (e) return e;
     }
     if (!g_batch_attr) {
-        e = cuda_check(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
+        e = cuda_check(cudaFuncSetAttribute(k_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
+        if (!e)
+            e = cuda_check(cudaFuncSetAttribute(k_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_TILE_SMEM + 4096), "attr");
         if (e) return e;
         g_batch_attr = true;
     }
@@ -702,7 +769,8 @@ int tg_batch_run(void *p, void *arena, int blocks, int window, uint32_t *values,
     A.spin_limit = g_batch_spin ? g_batch_spin : 20000000ull;   // about 2.5 s of polling by default
     int grid = blocks > 0 ? blocks : sm_count();
     if (finished < (unsigned)B.nplans) {
-        k_batch<<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
+        if (8 * B.nother > B.ngran) k_batch<true><<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
+        else k_batch<false><<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
         e = cuda_check(cudaGetLastError(), "batch launch");
         if (e) return e;
     }
@@ -831,6 +899,12 @@ static int server_submit(Server &S, const DensePlan &P) {
         R.value = 0;
         return (int)slot;
     }
+    int64_t ngran = 0, nother = 0;
+    for (const Seg &G : P.segs) {
+        ngran += G.kind == 4;
+        nother += G.kind == 1 && G.pp.nupd > 0;
+    }
+    S.fast |= 8 * nother > ngran;
     // parameter blob and jobs
     std::vector<uint8_t> prm;
     std::vector<BJob> jobs(P.segs.size());

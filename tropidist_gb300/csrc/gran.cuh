@@ -59,7 +59,8 @@ struct GranParams {
     uint32_t fin, fout;              // constant parts of the offsets (granules)
     uint32_t smask0, smask1;         // coset-number bits flipping in-granule bit 0 / 1 of the output
     GranOp ops[GP_MAXOPS];
-    uint4 min[GP_MEMBERS];           // member z: input offset, unpack selectors (even, odd lanes)
+    uint32_t xin[GP_MEMBERS];        // member z: input offset
+    uint2 usel[GP_MEMBERS];          // member z: unpack selectors (even, odd lanes)
     uint2 mout[GP_MEMBERS];          // member z: output offset, pack selector
     uint2 klow[8];                   // (input, output) offsets of coset-number bits 0 .. 7
     uint2 khigh[6][16];              // offsets of bits 8 + 4 g .. 11 + 4 g, by their value
@@ -288,19 +289,23 @@ static __device__ __forceinline__ void gran_step(const GranParams &P, uint32_t s
     for (int g = 0; g <= 5; g++) {
         if (g > nload) break;
 #pragma unroll
-        for (int z = (g ? 1 << (g - 1) : 0); z < (1 << g); z++) R[NQ * z] = __ldcg(in + (io ^ P.min[z].x));
+        for (int z = (g ? 1 << (g - 1) : 0); z < (1 << g); z++) R[NQ * z] = __ldcg(in + (io ^ P.xin[z]));
     }
+    // parameters in shared memory are read where they are used (as constants they are operands): read ahead
+    // they would take the registers that the members need
+    asm volatile("" ::: "memory");
 #pragma unroll
     for (int g = 0; g <= 5; g++) {
         if (g > nload) break;
 #pragma unroll
         for (int z = (g ? 1 << (g - 1) : 0); z < (1 << g); z++) {
             const uint32_t w = R[NQ * z];
-            R[NQ * z] = __byte_perm(w, 0u, P.min[z].y);
-            if (EB == 1) R[NQ * z + NQ - 1] = __byte_perm(w, 0u, P.min[z].z);
+            R[NQ * z] = __byte_perm(w, 0u, P.usel[z].x);
+            if (EB == 1) R[NQ * z + NQ - 1] = __byte_perm(w, 0u, P.usel[z].y);
         }
     }
     g_run_ops<EB>(P, k, R);
+    asm volatile("" ::: "memory");
     // output: in-granule permutation of the member, and of the thread's coset
     uint32_t ts;
     if (EB == 1) ts = ((__popc(k & P.smask0) & 1) ? 0x4444u : 0u) ^ ((__popc(k & P.smask1) & 1) ? 0x2222u : 0u);

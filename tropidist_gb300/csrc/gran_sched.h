@@ -246,7 +246,8 @@ static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, in
         for (int s = 0; s < L; s++)
             if ((z >> s) & 1u) o ^= dir[s];
         const uint32_t sh = (uint32_t)(o & lowm);
-        gp.min[z] = make_uint4((uint32_t)(o >> G), unpack_sel(sh, 0), unpack_sel(sh, 1), 0u);
+        gp.xin[z] = (uint32_t)(o >> G);
+        gp.usel[z] = make_uint2(unpack_sel(sh, 0), unpack_sel(sh, 1));
     }
     // ---- the register program, following every row's value
     uint64_t alive = (1ull << w_in) - 1;
@@ -403,14 +404,14 @@ static void emulate_gran(const GranParams &P, const E *src, E *dst) {
         uint32_t V[32][4];
         memset(V, 0, sizeof(V));
         for (int z = 0; z < (1 << P.nload); z++) {
-            const E *g = src + (size_t)(io ^ P.min[z].x) * NE;
+            const E *g = src + (size_t)(io ^ P.xin[z]) * NE;
             const uint8_t *by = reinterpret_cast<const uint8_t *>(g);
             for (int q = 0; q < NE; q++) {
                 if (EB == 1) {
-                    const uint32_t sel = (q & 1) ? P.min[z].z : P.min[z].y;
+                    const uint32_t sel = (q & 1) ? P.usel[z].y : P.usel[z].x;
                     V[z][q] = by[(sel >> (8 * (q >> 1))) & 3u];
                 } else {
-                    V[z][q] = g[((P.min[z].y >> (8 * q)) & 3u) >> 1];
+                    V[z][q] = g[((P.usel[z].x >> (8 * q)) & 3u) >> 1];
                 }
             }
         }
