@@ -319,7 +319,8 @@ int tree_move(void *destination, const void *source, size_t bytes);
  * right) state per generator.  info: heights, steps, launches per run, pairs, arena entries,
  * leaves, joins, single-block steps, block-product joins.  gemm: rows (join, F, mb, nb, kb, mapoff)
  * of joins run as min-plus products of 2^mb left and 2^nb right rows of 2^F entries (2^kb of them),
- * with their offset and parent vectors DL, DR, DT, PA, PB, PT (uint32) at gmaps[mapoff].
+ * with their offset and parent vectors DL, DR, DT, PA, PB, PT (uint32) at gmaps[mapoff]; with 256 added
+ * to F the vectors GA, GB, TA, TB follow: left row GA x ^ TA t and right row GB y ^ TB t of product t.
  * small_pairs (< 0: default): heights of at most that many pairs run in one single-block launch;
  * rbits (< 0: default): at most 2^rbits pairs per thread.  run: target = HOST bit vector of a
  * particular solution (ceil(ncols / 64) words); *value = root entry. */

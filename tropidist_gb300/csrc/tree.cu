@@ -13,8 +13,9 @@
 // grouped by height, all joins of one height in one launch of
 //   - k_tree_small: one block runs a whole run of consecutive small heights (a few thousand
 //     pairs each, e.g. the long spine of a comb tree) with a block barrier between heights;
-//   - k_tree_gemm: a join whose parents cover every pair of child blocks, as a tiled min-plus
-//     matrix product of XOR-permuted child rows through shared memory;
+//   - k_tree_gemm: a join whose pairs of child blocks are a product up to a few couplings (almost all
+//     pairs of a large tree), as tiled min-plus matrix products of XOR-permuted child rows through
+//     shared memory;
 //   - k_tree_fill + k_tree_join for the other joins: lane groups of 2^F lanes per parent (F <= 4),
 //     a warp per parent (F >= 5), or per-thread Gray walks of 2^R pairs of one parent; when a
 //     parent's pairs span threads they are reduced across the warp and committed with atomicMin
@@ -319,11 +320,16 @@ __global__ void __launch_bounds__(TR_BS, 3) k_tree_join(const TJoin *joins, int 
 }
 
 // ---------------------------------------------------------------- joins as min-plus block products
-// When the kernel generators are the unit pairs (e_k, e_k) and every left block meets every right
-// block, parent p = PA a ^ PB b ^ PT t reads left row a and right row b (2^F entries each) with
-// XOR offsets DL a and DR b ^ DT t, and its value is min over f of L'[a][f] + R'[b][f]: a min-plus
-// matrix product, tiled through shared memory (a 64 x 64 tile of parents per block, 16 per thread,
-// K in chunks of 32 staged with the offsets applied), every parent written once.
+// When the kernel generators are the unit pairs (e_k, e_k), parent p = PA x ^ PB y ^ PT t reads left row
+// GA x ^ TA t and right row GB y ^ TB t (2^F entries each) with XOR offsets DL x and DR y ^ DT t: for each
+// t the rows of one side meet all rows of the other (where every left block meets every right one the
+// rows are x and y themselves).  The value is min over f of L'[x][f] + R'[y][f]: a min-plus matrix
+// product, tiled through shared memory (a 64 x 64 tile of parents per block, 16 per thread, K in chunks
+// of 32 staged with the offsets applied), every parent written once.
+// A tile reads a child entry once for 64 pairs where the per-pair kernel reads two entries a pair: a
+// 240-column tree with joins of 2^31 to 2^33 pairs takes 2.35 ms for 4 targets, 4.65 ms with products
+// only where every block meets every other.  Joins of fewer than 64 rows on a side or of F < 2 stay
+// with the per-pair kernel (2^22 pairs at most on such trees).
 #define TG_T 64
 #define TG_KC 32
 #define TG_LD (TG_T + 4)
@@ -331,7 +337,9 @@ __global__ void __launch_bounds__(TR_BS, 3) k_tree_join(const TJoin *joins, int 
 struct TGemm {
     int64_t lo, ro, po;                // arena offsets of the left, right and parent tables
     int32_t F, mb, nb, kb;             // row length 2^F, 2^mb left rows, 2^nb right rows, 2^kb products
-    int32_t mapoff, pad;               // DL[mb] DR[nb] DT[kb] PA[mb] PB[nb] PT[kb] at gmaps[mapoff]
+    int32_t mapoff, rows;              // DL[mb] DR[nb] DT[kb] PA[mb] PB[nb] PT[kb] at gmaps[mapoff]; rows:
+                                       // then GA[mb] GB[nb] TA[kb] TB[kb], the rows that the tile's bits
+                                       // and the product's number stand for (else the rows themselves)
 };
 
 __device__ __forceinline__ uint32_t xor_bits(const uint32_t *v, int n, uint32_t x) {
@@ -380,8 +388,14 @@ __global__ void __launch_bounds__(256) k_tree_gemm(const __grid_constant__ TGemm
     // element j ^ (dl & (KC - 1))
     const int r = tid >> 2, q = tid & 3;
     const uint32_t dla = dl[r], drb = dr[r];
-    const uint32_t *Lrow = arena + G.lo + ((uint64_t)(a0 + r) << G.F);
-    const uint32_t *Rrow = arena + G.ro + ((uint64_t)(b0 + r) << G.F);
+    uint32_t la = a0 + r, rb = b0 + r;
+    if (G.rows) {
+        const uint32_t *GA = PT + G.kb, *GB = GA + G.mb, *TA = GB + G.nb, *TB = TA + G.kb;
+        la = xor_bits(GA, G.mb, la) ^ xor_bits(TA, G.kb, t);
+        rb = xor_bits(GB, G.nb, rb) ^ xor_bits(TB, G.kb, t);
+    }
+    const uint32_t *Lrow = arena + G.lo + ((uint64_t)la << G.F);
+    const uint32_t *Rrow = arena + G.ro + ((uint64_t)rb << G.F);
     const uint32_t nk = 1u << G.F, km = (uint32_t)KC - 1u;
     uint32_t xa[NE], yb[NE];
     auto fetch = [&](uint32_t k0) {
@@ -662,15 +676,27 @@ void *tg_tree_plan(const int64_t *leaves, int64_t nleaves, const int64_t *joins,
     std::vector<int> gemm_of((size_t)njoins, -1);
     for (int64_t g = 0; g < ngemm && st == TG_OK; g++) {
         const int64_t *r = gemm + 6 * g;
-        const int64_t j = r[0], F = r[1], mb = r[2], nb = r[3], kb = r[4], mo = r[5];
-        if (j < 0 || j >= njoins || gemm_of[j] >= 0 || F < 2 || F > 30 || mb < 6 || mb > 21 || nb < 6 || nb > 21 ||
-            kb < 0 || kb > 16 || mo < 0 || mo + 2 * (mb + nb + kb) > ngmaps || hj[j].F != F ||
+        const int64_t j = r[0], F = r[1] & 255, rows = r[1] >> 8, mb = r[2], nb = r[3], kb = r[4], mo = r[5];
+        const int64_t nm = rows ? 3 * (mb + nb) + 4 * kb : 2 * (mb + nb + kb);
+        if (rows < 0 || rows > 1 || j < 0 || j >= njoins || gemm_of[j] >= 0 || F < 2 || F > 30 || mb < 6 || mb > 21 ||
+            nb < 6 || nb > 21 || kb < 0 || kb > 16 || mo < 0 || mo + nm > ngmaps || hj[j].F != F ||
             hj[j].P != mb + nb + kb) {
             st = set_error(TG_ERR_ARG, "bad tree gemm row");
             break;
         }
-        const int64_t lsz = 1ll << (mb + F), rsz = 1ll << (nb + F);
-        if (hj[j].lo + lsz > arena || hj[j].ro + rsz > arena || (hj[j].lo & 7) || (hj[j].ro & 7))
+        int64_t lsz = 1ll << (mb + F), rsz = 1ll << (nb + F);
+        if (rows) {                        // the rows that the maps can reach
+            const uint32_t *GA = gmaps + mo + 2 * (mb + nb + kb), *GB = GA + mb, *TA = GB + nb, *TB = TA + kb;
+            uint64_t oa = 0, ob = 0;
+            for (int64_t k = 0; k < mb; k++) oa |= GA[k];
+            for (int64_t k = 0; k < nb; k++) ob |= GB[k];
+            for (int64_t k = 0; k < kb; k++) { oa |= TA[k]; ob |= TB[k]; }
+            lsz = rsz = 1ll << F;
+            for (; oa && lsz <= arena; oa >>= 1) lsz <<= 1;
+            for (; ob && rsz <= arena; ob >>= 1) rsz <<= 1;
+        }
+        if (lsz > arena || rsz > arena || hj[j].lo + lsz > arena || hj[j].ro + rsz > arena || (hj[j].lo & 7) ||
+            (hj[j].ro & 7))
             st = set_error(TG_ERR_ARG, "tree gemm reads outside the arena");
         for (int64_t k = 0; k < mb + nb + kb && st == TG_OK; k++) {       // offsets below 2^F, parents below 2^P
             if (gmaps[mo + k] >> F) st = set_error(TG_ERR_ARG, "tree gemm offset out of range");
@@ -679,7 +705,7 @@ void *tg_tree_plan(const int64_t *leaves, int64_t nleaves, const int64_t *joins,
         TGemm G;
         G.lo = hj[j].lo; G.ro = hj[j].ro; G.po = hj[j].po;
         G.F = (int32_t)F; G.mb = (int32_t)mb; G.nb = (int32_t)nb; G.kb = (int32_t)kb;
-        G.mapoff = (int32_t)mo; G.pad = 0;
+        G.mapoff = (int32_t)mo; G.rows = (int32_t)rows;
         gemm_of[j] = (int)T->hg.size();
         T->hg.push_back(G);
     }

@@ -31,6 +31,7 @@ import numpy as np
 
 DEFAULT_MEMORY_BYTES = 256 << 20       # cdist/tree_dp.py:40-41: the same limits, the same accounting
 DEFAULT_JOIN_WORK = 100_000_000
+GEMM_ROWS = 256                        # flag of a block product with row maps (tg_tree_plan)
 DEVICE_INDEX_BITS = 32                 # device tables are indexed by uint32 states
 
 
@@ -481,8 +482,8 @@ class CompiledTreeDP:
                 nd, jn = self.nodes[i], self.joins[i]
                 g = gemm_form(jn)
                 if g is not None and g["F"] >= 2 and 6 <= g["mb"] <= 21 and 6 <= g["nb"] <= 21 and g["kb"] <= 16:
-                    grows.append([len(rows), g["F"], g["mb"], g["nb"], g["kb"], len(gmaps)])
-                    for k in ("DL", "DR", "DT", "PA", "PB", "PT"):
+                    grows.append([len(rows), g["F"] | GEMM_ROWS, g["mb"], g["nb"], g["kb"], len(gmaps)])
+                    for k in ("DL", "DR", "DT", "PA", "PB", "PT", "GA", "GB", "TA", "TB"):
                         gmaps.extend(g[k])
                 rows.append([off[nd.left], off[nd.right], off[i], jn.parent_rank, len(jn.free_maps), h,
                              len(maps) // 2, 0])
@@ -645,32 +646,76 @@ def gemm_form(join):
     """The block-product form of a join, or None.
 
     With the kernel generators (e_k, e_k), parent p reads left entries (a(p) << F) | f and right
-    entries (b(p) << F) | (f ^ d(p)) for f < 2^F, where a, b, d are linear in p.  When p -> (a, b)
-    is onto (every left block meets every right block), p = PA a ^ PB b ^ PT t with t in the kernel of
-    that map, and d = DL a ^ DR b ^ DT t; with f' = f ^ DL a the parent's value is
-        min over f' of L[(a << F) | (f' ^ DL a)] + R[(b << F) | (f' ^ DR b ^ DT t)]
+    entries (b(p) << F) | (f ^ d(p)) for f < 2^F, where a, b, d are linear in p.  The image S of
+    p -> (a, b) holds left parts SA = {(a, 0)} and right parts SB = {(0, b)} (mb and nb dimensions) and
+    a complement of couplings (a, b); with a basis GA of SA, GB of SB, and t over the couplings and the
+    kernel of p -> (a, b) (kb dimensions),
+        p = PA x ^ PB y ^ PT t,  a = GA x ^ TA t,  b = GB y ^ TB t,  d = DL x ^ DR y ^ DT t
+    and with f' = f ^ DL x the parent's value is
+        min over f' of L[(a << F) | (f' ^ DL x)] + R[(b << F) | (f' ^ DR y ^ DT t)]
     a min-plus product of 2^mb left rows and 2^nb right rows of length 2^F, once per t.
-    Returns dict(F, mb, nb, kb, DL, DR, DT, PA, PB, PT) (lists of ints, one per bit)."""
+    Returns dict(F, mb, nb, kb, DL, DR, DT, PA, PB, PT, GA, GB, TA, TB) (lists of ints, one per bit); GA
+    and GB are the unit vectors and TA, TB zero where every left block meets every right block."""
     F = len(join.free_maps)
     lr, rr, P = join.left_rank, join.right_rank, join.parent_rank
-    mb, nb = lr - F, rr - F
+    wl, wr = lr - F, rr - F
     low = (1 << F) - 1
-    # per parent generator: its (a | b << mb) block coordinates and its d
+    # per parent generator: its (a | b << wl) block coordinates and its d
     ab, dd = [], []
     for m in join.parent_maps:
         left, right = m & ((1 << lr) - 1), m >> lr
         if left & low:
             return None
-        ab.append((left >> F) | ((right >> F) << mb))
+        ab.append((left >> F) | ((right >> F) << wl))
         dd.append(right & low)
     e = _Eliminator(track=True)
     for v in ab:
         e.add(v)
-    if e.rank() != mb + nb:
-        return None
-    PA = [e.express(1 << i) for i in range(mb)]
-    PB = [e.express(1 << (mb + j)) for j in range(nb)]
-    PT = list(e.dependencies)
+    lmask = (1 << wl) - 1
+    kernel = list(e.dependencies)
+    if e.rank() == wl + wr:
+        GA, GB, couplings = [1 << i for i in range(wl)], [1 << j for j in range(wr)], []
+        PA = [e.express(g) for g in GA]
+        PB = [e.express(g << wl) for g in GB]
+    else:
+        # SA: combinations of the image's vectors whose right part vanishes; SB likewise; the couplings are
+        # vectors of the image outside SA + SB
+        SA, SB = _vanishing(ab, lambda v: v >> wl), _vanishing(ab, lambda v: v & lmask)
+        PA, GA = [c for c, _ in SA], [v & lmask for _, v in SA]
+        PB, GB = [c for c, _ in SB], [v >> wl for _, v in SB]
+        span = _Eliminator()
+        for g in GA:
+            span.add(g)
+        for g in GB:
+            span.add(g << wl)
+        couplings = []
+        for i, v in enumerate(ab):
+            before = span.rank()
+            span.add(v)
+            if span.rank() > before:
+                couplings.append(1 << i)
+    PT = kernel + couplings
     d_of = lambda comb: _combine(dd, comb)
-    return {"F": F, "mb": mb, "nb": nb, "kb": len(PT), "PA": PA, "PB": PB, "PT": PT,
-            "DL": [d_of(c) for c in PA], "DR": [d_of(c) for c in PB], "DT": [d_of(c) for c in PT]}
+    v_of = lambda comb: _combine(ab, comb)
+    TA, TB = [v_of(c) & lmask for c in PT], [v_of(c) >> wl for c in PT]
+    if len(PA) + len(PB) + len(PT) != P:
+        return None
+    return {"F": F, "mb": len(PA), "nb": len(PB), "kb": len(PT), "PA": PA, "PB": PB, "PT": PT,
+            "DL": [d_of(c) for c in PA], "DR": [d_of(c) for c in PB], "DT": [d_of(c) for c in PT],
+            "GA": GA, "GB": GB, "TA": TA, "TB": TB}
+
+
+def _vanishing(vectors, part):
+    """A basis of the combinations of `vectors` that are nonzero and whose part(v) is 0, as (combination,
+    value) pairs: the dependencies of the parts, reduced by their values."""
+    e = _Eliminator(track=True)
+    for v in vectors:
+        e.add(part(v))
+    out, seen = [], _Eliminator()
+    for comb in e.dependencies:
+        v = _combine(vectors, comb)
+        before = seen.rank()
+        seen.add(v)
+        if seen.rank() > before:
+            out.append((comb, v))
+    return out
