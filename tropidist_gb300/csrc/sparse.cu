@@ -99,6 +99,105 @@ __device__ __forceinline__ uint32_t sp_lookup(const unsigned long long *H, int l
     return 255;
 }
 
+// the rest of an insertion whose compare-and-swap at its first slot i returned prev; -1 if full
+__device__ __forceinline__ int sp_insert_rest(unsigned long long *H, int lg, uint32_t i, unsigned long long prev,
+                                              unsigned long long packed) {
+    if (prev == SP_EMPTY) return 1;
+    const uint32_t mask = (1u << lg) - 1u;
+    for (uint32_t probe = 0; probe < mask; probe++) {
+        if (((prev ^ packed) & SP_KEYMASK) == 0) {
+            if (packed < prev) atomicMin(H + i, packed);
+            return 0;
+        }
+        i = (i + 1) & mask;
+        prev = atomicCAS(H + i, SP_EMPTY, packed);
+        if (prev == SP_EMPTY) return 1;
+    }
+    if (((prev ^ packed) & SP_KEYMASK) == 0) {
+        if (packed < prev) atomicMin(H + i, packed);
+        return 0;
+    }
+    return -1;
+}
+
+// sp_insert_min without the load before the claim, for keys that are mostly new
+__device__ __forceinline__ int sp_insert_new(unsigned long long *H, int lg, uint64_t key, uint32_t v) {
+    const unsigned long long packed = key | ((unsigned long long)v << 56);
+    const uint32_t i = sp_slot(key, lg);
+    return sp_insert_rest(H, lg, i, atomicCAS(H + i, SP_EMPTY, packed), packed);
+}
+
+// One state of a walk's table through its column: the state itself and its neighbour over the column's
+// update, each inserted into the next index where the select, the cap and the bound let it through.  The
+// accesses of the two are issued together (the old index at the neighbour's key beside the state's claim,
+// the claims without a load before them), so a state waits two round trips where it waited five.
+// With sp_compact, the walks of a query of 3048 columns at K = 6 (tables of up to 8192 states, L2): 198 ms
+// where the chained accesses and a claim per slot took 415; of 5000 columns in shared memory: 138, 202.
+// Returns whether the neighbour improved on the old table (chg: its entry).
+struct SpStep {
+    uint64_t upd, selm, selb;
+    int cap, kb, w;
+    bool want;
+};
+
+__device__ __forceinline__ bool sp_step_state(const SpStep &s, const BoundParams &B, unsigned long long x,
+                                              const unsigned long long *curH, int lg, unsigned long long *H, int lgn,
+                                              unsigned long long &chg, bool &full) {
+    const uint64_t key = x & SP_KEYMASK, clr = ~s.selm & SP_KEYMASK, t = key ^ s.upd;
+    const uint32_t v = (uint32_t)(x >> 56), vc = v + (uint32_t)s.w;
+    const uint64_t k2 = key & clr, t2 = t & clr;
+    const bool in1 = (key & s.selm) == s.selb && (int)v <= s.cap && sp_keep(B, k2, v);
+    bool in2 = s.upd && (int)v < s.cap && (t & s.selm) == s.selb && (int)vc <= s.cap && sp_keep(B, t2, vc);
+    const unsigned long long p1 = k2 | ((unsigned long long)v << 56), p2 = t2 | ((unsigned long long)vc << 56);
+    const uint32_t i1 = sp_slot(k2, lgn), i2 = sp_slot(t2, lgn), mask = (1u << lg) - 1u;
+    uint32_t j = sp_slot(t, lg);
+    unsigned long long old = SP_EMPTY, r1 = SP_EMPTY, r2 = SP_EMPTY;
+    if (in2 && curH) old = curH[j];
+    if (in1) r1 = atomicCAS(H + i1, SP_EMPTY, p1);
+    bool changed = false;
+    chg = p2;
+    if (in2) {
+        for (uint32_t probe = 0; probe < mask && old != SP_EMPTY && ((old ^ t) & SP_KEYMASK); probe++) {
+            j = (j + 1) & mask;
+            old = curH[j];
+        }
+        const uint32_t vo = old != SP_EMPTY && ((old ^ t) & SP_KEYMASK) == 0 ? (uint32_t)(old >> 56) : 255u;
+        changed = vc < vo && s.want;
+        in2 = vo != 255u || s.kb < 0 || (int)vc < s.kb;
+        if (in2) r2 = atomicCAS(H + i2, SP_EMPTY, p2);
+    }
+    if (in1 && sp_insert_rest(H, lgn, i1, r1, p1) < 0) full = true;
+    if (in2 && sp_insert_rest(H, lgn, i2, r2, p2) < 0) full = true;
+    return changed;
+}
+
+// The filled slots of an index into a list, by all threads of the block (2^lg and the block's threads are
+// multiples of a warp): eight slots a thread in flight, one claim of list positions per warp for them.
+__device__ __forceinline__ void sp_compact(const unsigned long long *H, uint32_t cap, unsigned long long *A,
+                                           unsigned long long *ctr, unsigned tid, unsigned NT) {
+    const unsigned lane = tid & 31u, below = (1u << lane) - 1u;
+    for (uint32_t k0 = tid; k0 < cap; k0 += 8 * NT) {
+        unsigned long long x[8];
+        unsigned bal[8], tot = 0;
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = k0 + u * NT < cap ? H[k0 + u * NT] : SP_EMPTY;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            bal[u] = __ballot_sync(0xffffffffu, x[u] != SP_EMPTY);
+            tot += __popc(bal[u]);
+        }
+        if (!tot) continue;
+        unsigned long long q = 0;
+        if (lane == 0) q = atomicAdd(ctr, (unsigned long long)tot);
+        q = __shfl_sync(0xffffffffu, q, 0);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (x[u] != SP_EMPTY) A[q + __popc(bal[u] & below)] = x[u];
+            q += __popc(bal[u]);
+        }
+    }
+}
+
 __global__ void k_sp_fill(unsigned long long *H, uint64_t n) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         H[i] = SP_EMPTY;
@@ -359,7 +458,7 @@ __host__ __device__ static int lg_tiny(uint64_t m) {
 
 // ---- tables that fit shared memory: the same steps with the old table, the new one and the changed list
 // there, so that index probes and claims are shared-memory atomics: from the global scratch one SM's
-// random L2 atomics bound the step (25 us a step at 1000 states; 13 us here, host included).  It takes tables of at most SPW_TINY_N / 2
+// random L2 atomics bound the step.  It takes tables of at most SPW_TINY_N / 2
 // states and stops (reason 1) when a step would need more.  The next step's row is fetched during this
 // one.  A kept table is a plain copy of its states and of the working index (load 1/4 to 1/2), unless
 // that index is more than twice what the table needs.  The truncated table of a cut takes the old
@@ -414,7 +513,7 @@ __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_
         for (unsigned k = tid; k < n; k += NT) {
             const unsigned long long x = P.A0[k];
             sA(0)[k] = x;
-            if (sp_insert_min(sH(0), lg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+            if (sp_insert_new(sH(0), lg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
         }
     }
     __syncthreads();
@@ -429,34 +528,17 @@ __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_
         const unsigned long long *curA = sA(sl), *curH = sH(sl);
         unsigned long long *H = sH(sl ^ 1), *A = sA(sl ^ 1);
         if (tid < 3) c_cnt[b ^ 1][tid] = 0;              // read last before the barrier that ended step i - 1
-        const uint64_t upd = (uint64_t)f[SW_UPD] & SP_KEYMASK, selm = (uint64_t)f[SW_SELM], selb = (uint64_t)f[SW_SELB];
-        const uint64_t clr = ~selm & SP_KEYMASK;
-        const int cap = (int)f[SW_CAP], kb = (int)f[SW_KB], w = (int)f[SW_W];
         const bool want = f[SW_WANT] != 0;
+        const SpStep st = {(uint64_t)f[SW_UPD] & SP_KEYMASK, (uint64_t)f[SW_SELM], (uint64_t)f[SW_SELB],
+                           (int)f[SW_CAP], (int)f[SW_KB], (int)f[SW_W], want};
         for (unsigned k0 = 0; k0 < n; k0 += NT) {
             const unsigned k = k0 + tid;
             unsigned long long chg = 0;
             bool changed = false;
             if (k < n) {
-                const unsigned long long x = curA[k];
-                const uint64_t key = x & SP_KEYMASK;
-                const uint32_t v = (uint32_t)(x >> 56);
-                if ((key & selm) == selb) {
-                    const uint64_t k2 = key & clr;
-                    if ((int)v <= cap && sp_keep(B, k2, v) && sp_insert_min(H, lgn, k2, v) < 0) atomicOr(&c_flag, 1ull);
-                }
-                if (upd && (int)v < cap) {
-                    const uint64_t t = key ^ upd;
-                    const uint32_t vc = v + (uint32_t)w;
-                    const uint64_t t2 = t & clr;
-                    if ((t & selm) == selb && (int)vc <= cap && sp_keep(B, t2, vc)) {
-                        const uint32_t vo = sp_lookup(curH, lg, t);
-                        changed = vc < vo && want;
-                        chg = t2 | ((unsigned long long)vc << 56);
-                        if ((vo != 255u || kb < 0 || (int)vc < kb) && sp_insert_min(H, lgn, t2, vc) < 0)
-                            atomicOr(&c_flag, 1ull);
-                    }
-                }
+                bool full = false;
+                changed = sp_step_state(st, B, curA[k], curH, lg, H, lgn, chg, full);
+                if (full) atomicOr(&c_flag, 1ull);
             }
             if (want) {
                 __syncwarp();
@@ -466,11 +548,7 @@ __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_
         }
         if (i + 1 < P.nsteps) load_row(i + 1, b ^ 1);
         __syncthreads();
-        for (unsigned k = tid; k < capn; k += NT) {      // capn and NT are multiples of the warp
-            const unsigned long long x = H[k];
-            const unsigned long long q = sp_claim(&cnt[1], x != SP_EMPTY);
-            if (x != SP_EMPTY) A[q] = x;                 // at most 2 n
-        }
+        sp_compact(H, (uint32_t)capn, A, &cnt[1], tid, NT);
         __syncthreads();
         if (c_flag) { reason = 4; break; }
         uint64_t nn = cnt[1];
@@ -501,7 +579,7 @@ __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_
                 const unsigned k = k0 + tid;
                 const unsigned long long x = k < nn ? A[k] : SP_EMPTY;
                 const bool in = k < nn && (int)(x >> 56) < below;
-                if (in && sp_insert_min(T, nlg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                if (in && sp_insert_new(T, nlg, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
                 __syncwarp();
                 const unsigned long long q = sp_claim(&cnt[2], in);
                 if (in) TA[q] = x;
@@ -550,7 +628,7 @@ __global__ void __launch_bounds__(SPW_TINY_THREADS) k_sp_walk_tiny(const __grid_
         if (kH)
             for (unsigned k = tid; k < n; k += NT) {
                 const unsigned long long x = sA(sl)[k];
-                if (sp_insert_min(kH, lgk, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                if (sp_insert_new(kH, lgk, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
             }
     }
     // the current table to a global scratch slot (not the one it came from)
@@ -624,34 +702,17 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __gri
         const uint64_t capn = 1ull << lgn;
         unsigned long long *H = P.idx[os], *A = P.arr[os];
         if (tid < 3) c_cnt[b ^ 1][tid] = 0;              // read last before the barrier that ended step i - 1
-        const uint64_t upd = (uint64_t)f[SW_UPD] & SP_KEYMASK, selm = (uint64_t)f[SW_SELM], selb = (uint64_t)f[SW_SELB];
-        const uint64_t clr = ~selm & SP_KEYMASK;
-        const int cap = (int)f[SW_CAP], kb = (int)f[SW_KB], w = (int)f[SW_W];
         const bool want = f[SW_WANT] != 0;
+        const SpStep st = {(uint64_t)f[SW_UPD] & SP_KEYMASK, (uint64_t)f[SW_SELM], (uint64_t)f[SW_SELB],
+                           (int)f[SW_CAP], (int)f[SW_KB], (int)f[SW_W], want};
         for (uint64_t k0 = 0; k0 < n; k0 += NT) {
             const uint64_t k = k0 + tid;
             unsigned long long chg = 0;
             bool changed = false;
             if (k < n) {
-                const unsigned long long x = curA[k];
-                const uint64_t key = x & SP_KEYMASK;
-                const uint32_t v = (uint32_t)(x >> 56);
-                if ((key & selm) == selb) {
-                    const uint64_t k2 = key & clr;
-                    if ((int)v <= cap && sp_keep(B, k2, v) && sp_insert_min(H, lgn, k2, v) < 0) atomicOr(&c_flag, 1ull);
-                }
-                if (upd && (int)v < cap) {
-                    const uint64_t t = key ^ upd;
-                    const uint32_t vc = v + (uint32_t)w;
-                    const uint64_t t2 = t & clr;
-                    if ((t & selm) == selb && (int)vc <= cap && sp_keep(B, t2, vc)) {
-                        const uint32_t vo = sp_lookup(curH, lg, t);
-                        changed = vc < vo && want;
-                        chg = t2 | ((unsigned long long)vc << 56);
-                        if ((vo != 255u || kb < 0 || (int)vc < kb) && sp_insert_min(H, lgn, t2, vc) < 0)
-                            atomicOr(&c_flag, 1ull);
-                    }
-                }
+                bool full = false;
+                changed = sp_step_state(st, B, curA[k], curH, lg, H, lgn, chg, full);
+                if (full) atomicOr(&c_flag, 1ull);
             }
             if (want) {
                 __syncwarp();
@@ -661,11 +722,7 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __gri
         }
         if (i + 1 < P.nsteps) load_row(i + 1, b ^ 1);
         __syncthreads();
-        for (uint64_t k = tid; k < capn; k += NT) {      // capn and NT are multiples of the warp
-            const unsigned long long x = H[k];
-            const unsigned long long q = sp_claim(&cnt[1], x != SP_EMPTY);
-            if (x != SP_EMPTY) A[q] = x;
-        }
+        sp_compact(H, (uint32_t)capn, A, &cnt[1], tid, NT);
         __syncthreads();
         if (c_flag) { reason = 4; break; }
         uint64_t nn = cnt[1];
@@ -699,7 +756,7 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __gri
                 const uint64_t k = k0 + tid;
                 const unsigned long long x = k < nn ? A[k] : SP_EMPTY;
                 const bool in = k < nn && (int)(x >> 56) < below;
-                if (in && sp_insert_min(T, lgt, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                if (in && sp_insert_new(T, lgt, x & SP_KEYMASK, (uint32_t)(x >> 56)) < 0) atomicOr(&c_flag, 1ull);
                 __syncwarp();
                 const unsigned long long q = sp_claim(&cnt[2], in);
                 if (in) TA[q] = x;
@@ -746,7 +803,7 @@ __global__ void __launch_bounds__(SPW_SMALL_THREADS) k_sp_walk_small(const __gri
         __syncthreads();
         if (kH)
             for (uint64_t k = tid; k < n; k += NT)
-                if (sp_insert_min(kH, lgk, curA[k] & SP_KEYMASK, (uint32_t)(curA[k] >> 56)) < 0) atomicOr(&c_flag, 1ull);
+                if (sp_insert_new(kH, lgk, curA[k] & SP_KEYMASK, (uint32_t)(curA[k] >> 56)) < 0) atomicOr(&c_flag, 1ull);
     }
     if (tid == 0) {
         P.state[0] = (unsigned long long)i;
