@@ -74,12 +74,18 @@ __device__ __forceinline__ void spw_load(const uint64_t *keys, uint64_t stride, 
     for (int w = 0; w < W; w++) k[w] = keys[(uint64_t)w * stride + i];
 }
 
-// key words written by other threads of the same launch: read through L2
-template <int W>
-__device__ __forceinline__ bool spw_equal_cg(const uint64_t *keys, uint64_t stride, uint64_t i, const uint64_t (&k)[W]) {
+// a word written by other threads of the same launch: read through L2, or from the block's shared memory
+template <bool SM, typename T>
+__device__ __forceinline__ T spw_ld(const T *p) {
+    if constexpr (SM) return *p;
+    else return __ldcg(p);
+}
+
+template <int W, bool SM>
+__device__ __forceinline__ bool spw_equal(const uint64_t *keys, uint64_t stride, uint64_t i, const uint64_t (&k)[W]) {
     bool eq = true;
 #pragma unroll
-    for (int w = 0; w < W; w++) eq = eq && __ldcg(keys + (uint64_t)w * stride + i) == k[w];
+    for (int w = 0; w < W; w++) eq = eq && spw_ld<SM>(keys + (uint64_t)w * stride + i) == k[w];
     return eq;
 }
 
@@ -98,16 +104,16 @@ __device__ __forceinline__ bool spw_keep(const WideBound &b, const uint64_t (&k)
 }
 
 // value of key in a table's index (255 when absent)
-template <int W>
+template <int W, bool SM = false>
 __device__ __forceinline__ uint32_t spw_lookup(const unsigned long long *H, int lg, const uint64_t *keys,
                                                uint64_t stride, const uint64_t (&k)[W]) {
     if (!H) return 255u;
     const uint32_t mask = (1u << lg) - 1u;
     uint32_t s = spw_slot<W>(k, lg);
     for (uint32_t probe = 0; probe <= mask; probe++) {
-        const unsigned long long cur = __ldcg(H + s);
+        const unsigned long long cur = spw_ld<SM>(H + s);
         if (cur == SPW_EMPTY) return 255u;
-        if (spw_equal_cg<W>(keys, stride, cur & SPW_IDX, k)) return (uint32_t)(cur >> 56);
+        if (spw_equal<W, SM>(keys, stride, cur & SPW_IDX, k)) return (uint32_t)(cur >> 56);
         s = (s + 1) & mask;
     }
     return 255u;
@@ -125,29 +131,36 @@ __device__ __forceinline__ Lanes grid_lanes() {
 }
 __device__ __forceinline__ Lanes block_lanes() { return Lanes{threadIdx.x, blockDim.x, 0, blockDim.x}; }
 
-// staging: write the key, then insert value << 56 | e keeping the least word per key (BLK: all
-// writers and readers are threads of one block)
-template <int W, bool BLK>
-__device__ __forceinline__ void spw_emit(uint64_t *ek, uint64_t estride, uint8_t *ev, unsigned long long *H, int lg,
-                                         uint64_t e, const uint64_t (&k)[W], uint32_t v, unsigned long long *err) {
+// staging: write the key and its value at position e
+template <int W, bool SM>
+__device__ __forceinline__ void spw_stage(uint64_t *ek, uint64_t estride, uint8_t *ev, uint64_t e,
+                                          const uint64_t (&k)[W], uint32_t v) {
 #pragma unroll
-    for (int w = 0; w < W; w++) __stcg(ek + (uint64_t)w * estride + e, k[w]);
+    for (int w = 0; w < W; w++) {
+        if constexpr (SM) ek[(uint64_t)w * estride + e] = k[w];
+        else __stcg(ek + (uint64_t)w * estride + e, k[w]);
+    }
     ev[e] = (uint8_t)v;
-    if (BLK) __threadfence_block();
-    else __threadfence();
-    const unsigned long long word = ((unsigned long long)v << 56) | e;
+}
+
+// the rest of an insertion whose compare-and-swap at its first slot s returned cur: the least word per key
+// stays (BLK: all writers and readers are threads of one block, SM: in its shared memory)
+template <int W, bool BLK, bool SM>
+__device__ __forceinline__ void spw_insert_rest(const uint64_t *ek, uint64_t estride, unsigned long long *H, int lg,
+                                                uint32_t s, unsigned long long cur, const uint64_t (&k)[W],
+                                                unsigned long long word, unsigned long long *err) {
     const uint32_t mask = (1u << lg) - 1u;
-    uint32_t s = spw_slot<W>(k, lg);
     for (uint32_t probe = 0; probe <= mask; probe++) {
-        unsigned long long cur = atomicCAS(H + s, SPW_EMPTY, word);
         if (cur == SPW_EMPTY) return;
         if (BLK) __threadfence_block();
         else __threadfence();
-        if (spw_equal_cg<W>(ek, estride, cur & SPW_IDX, k)) {
+        if (spw_equal<W, SM>(ek, estride, cur & SPW_IDX, k)) {
             atomicMin(H + s, word);
             return;
         }
+        if (probe == mask) break;
         s = (s + 1) & mask;
+        cur = atomicCAS(H + s, SPW_EMPTY, word);
     }
     atomicOr(err, 1ull);
 }
@@ -166,7 +179,7 @@ __device__ __forceinline__ uint64_t spw_count(const unsigned long long *n_dev, u
 }
 
 // every old state and its candidate through the column into the staging index
-template <int W, bool BLK>
+template <int W, bool BLK, bool SM = false>
 __device__ __forceinline__ void spw_emit_body(const Lanes &L, const uint64_t *__restrict__ keys,
                                               const uint8_t *__restrict__ vals, uint64_t n, uint64_t stride,
                                               uint64_t *ek, uint8_t *ev, uint64_t estride, unsigned long long *H,
@@ -176,32 +189,34 @@ __device__ __forceinline__ void spw_emit_body(const Lanes &L, const uint64_t *__
         uint64_t k[W];
         spw_load<W>(keys, stride, i, k);
         const uint32_t v = vals[i];
-        // the old state
-        bool pass = true;
+        // the old state and its candidate: both staged before one fence, both claims in flight together
+        uint64_t c1[W], c2[W];
+        bool in1 = true, in2 = true, any = false;
 #pragma unroll
-        for (int w = 0; w < W; w++) pass = pass && (k[w] & P.sel_mask[w]) == P.sel_bits[w];
-        if (pass) {
-            uint64_t c[W];
-#pragma unroll
-            for (int w = 0; w < W; w++) c[w] = k[w] & ~P.sel_mask[w];
-            if ((int)v <= P.cap && spw_keep<W>(B, c, v))
-                spw_emit<W, BLK>(ek, estride, ev, H, lg, 2 * i, c, v, counters + 2);
+        for (int w = 0; w < W; w++) {
+            const uint64_t t = k[w] ^ P.upd[w];
+            any = any || P.upd[w] != 0;
+            in1 = in1 && (k[w] & P.sel_mask[w]) == P.sel_bits[w];
+            in2 = in2 && (t & P.sel_mask[w]) == P.sel_bits[w];
+            c1[w] = k[w] & ~P.sel_mask[w];
+            c2[w] = t & ~P.sel_mask[w];
         }
-        // its candidate
-        if ((int)v < P.cap && (int)v + P.w <= P.cap) {
-            uint64_t c[W];
-            bool cpass = true, any = false;
-#pragma unroll
-            for (int w = 0; w < W; w++) {
-                c[w] = k[w] ^ P.upd[w];
-                any = any || P.upd[w] != 0;
-                cpass = cpass && (c[w] & P.sel_mask[w]) == P.sel_bits[w];
-                c[w] &= ~P.sel_mask[w];
-            }
-            const uint32_t cv = v + (uint32_t)P.w;
-            if (any && cpass && spw_keep<W>(B, c, cv))
-                spw_emit<W, BLK>(ek, estride, ev, H, lg, 2 * i + 1, c, cv, counters + 2);
-        }
+        const uint32_t cv = v + (uint32_t)P.w;
+        in1 = in1 && (int)v <= P.cap && spw_keep<W>(B, c1, v);
+        in2 = in2 && any && (int)v < P.cap && (int)cv <= P.cap && spw_keep<W>(B, c2, cv);
+        if (!in1 && !in2) continue;
+        if (in1) spw_stage<W, SM>(ek, estride, ev, 2 * i, c1, v);
+        if (in2) spw_stage<W, SM>(ek, estride, ev, 2 * i + 1, c2, cv);
+        if (BLK) __threadfence_block();
+        else __threadfence();
+        const unsigned long long w1 = ((unsigned long long)v << 56) | (2 * i);
+        const unsigned long long w2 = ((unsigned long long)cv << 56) | (2 * i + 1);
+        const uint32_t s1 = spw_slot<W>(c1, lg), s2 = spw_slot<W>(c2, lg);
+        unsigned long long r1 = SPW_EMPTY, r2 = SPW_EMPTY;
+        if (in1) r1 = atomicCAS(H + s1, SPW_EMPTY, w1);
+        if (in2) r2 = atomicCAS(H + s2, SPW_EMPTY, w2);
+        if (in1) spw_insert_rest<W, BLK, SM>(ek, estride, H, lg, s1, r1, c1, w1, counters + 2);
+        if (in2) spw_insert_rest<W, BLK, SM>(ek, estride, H, lg, s2, r2, c2, w2, counters + 2);
     }
 }
 
@@ -218,7 +233,7 @@ __global__ void k_spw_emit(const uint64_t *__restrict__ keys, const uint8_t *__r
 
 // new table (keys, vals, index lg2) from the staging index; changed states from candidate slots.
 // Tiles of blockDim slots: output positions are claimed once per block and tile.
-template <int W>
+template <int W, bool SM = false>
 __device__ __forceinline__ void spw_compact_body(const Lanes &L, const unsigned long long *__restrict__ H,
                                                  uint64_t hcap, const uint64_t *__restrict__ ek, uint64_t estride,
                                                  uint64_t *nk, uint8_t *nv, uint64_t ncap, unsigned long long *H2,
@@ -235,7 +250,7 @@ __device__ __forceinline__ void spw_compact_body(const Lanes &L, const unsigned 
 #pragma unroll
         for (int q = 0; q < SPW_PER; q++) {
             const uint64_t s = t0 + (uint64_t)q * blockDim.x + threadIdx.x;
-            const unsigned long long cur = s < hcap ? __ldcg(H + s) : SPW_EMPTY;
+            const unsigned long long cur = s < hcap ? spw_ld<SM>(H + s) : SPW_EMPTY;
             cw[q] = cur;
             if (cur == SPW_EMPTY) continue;
             const uint64_t e = cur & SPW_IDX;
@@ -248,7 +263,7 @@ __device__ __forceinline__ void spw_compact_body(const Lanes &L, const unsigned 
                 spw_load<W>(ek, estride, e, o);
 #pragma unroll
                 for (int w = 0; w < W; w++) o[w] |= P.sel_bits[w];
-                if (v < spw_lookup<W>(Hold, lg_old, okeys, ostride, o)) cmask |= 1u << q;
+                if (v < spw_lookup<W, SM>(Hold, lg_old, okeys, ostride, o)) cmask |= 1u << q;
             }
         }
         unsigned long long j, jc;
@@ -591,142 +606,242 @@ struct SpwSmall {
     const uint64_t *words, *masks;
     const int64_t *weights;
     int maxc, K, i0, nsteps, cur;
-    uint64_t cap, limit, arena_bytes;
+    uint64_t cap, limit, back, arena_bytes;          // back: stop (reason 5) once 4 n <= back
     SpwRing ring[3], sg, ch;
     unsigned long long *cnt, *res;
     uint64_t *resk;
     uint8_t *resv, *arena;
 };
 
-// Steps i0.. of a walk in one block while the tables are small (no launch per kernel of a step): the
-// same bodies as the separate kernels, with the block's barriers between them.  Stops before a step
-// whose table holds more than limit / 2 states (reason 1) or after a step that raised a flag (reason 4,
-// the walk is void); state: [0] next step, [1] ring slot of its table, [2] reason.
-//
-// Bound: the chain of dependent L2 accesses of a step (row, state, index probe, claim), not bytes.
-// The next step's row is fetched during this one, its indexes are cleared beside this step's kept copy,
-// and that copy is written while the next step's states go in.  Three-word states, host included: 20 to
-// 27 us a step at 300 to 1000 states, where the separate launches take 55 to 65 (host-bound); 17 us at
-// 10 states, before 25.
+// a block's copy of step i's parameters
 template <int W>
-__global__ void __launch_bounds__(SPW_SMALL_THREADS) k_spw_walk_small(const __grid_constant__ SpwSmall S) {
+__device__ __forceinline__ void spw_load_row(const SpwSmall &S, int i, WideStep &P, WideBound &B, uint64_t *jt) {
+    const int64_t *f = S.steps + (size_t)SPW_WALK_FIELDS * i;
+    const uint64_t *wd = S.words + (size_t)5 * W * i;
+    const int ncls = f[WK_USEH] ? (int)f[WK_NCLS] : 0;
+    if (threadIdx.x == 0) {
+        P.cap = (int)f[WK_CAP];
+        P.keep_below = (int)f[WK_KB];
+        P.w = (int)f[WK_W];
+        P.want_changed = f[WK_JOIN] != 0;
+        B.on = (int)f[WK_USEH];
+        B.ncls = ncls;
+        B.K = S.K;
+        B.extra = f[WK_EXTRA];
+    }
+    for (unsigned q = threadIdx.x; q < (unsigned)W; q += blockDim.x) {
+        P.upd[q] = wd[q];
+        P.sel_mask[q] = wd[W + q];
+        P.sel_bits[q] = wd[2 * W + q];
+        B.tmask[q] = wd[3 * W + q];
+        jt[q] = wd[4 * W + q];
+    }
+    for (unsigned c = threadIdx.x; c < (unsigned)(ncls * W); c += blockDim.x)
+        B.mask[c / W][c % W] = S.masks[((size_t)i * S.maxc) * W + c];
+    for (unsigned c = threadIdx.x; c < (unsigned)ncls; c += blockDim.x) B.w[c] = S.weights[(size_t)i * S.maxc + c];
+}
+
+#define SPW_SM_THREADS 512
+// states a table in shared memory may hold: two tables, the staging and the changed list (8 W + 1 bytes a
+// state) and three indexes (16 bytes a state) within 227 KB
+__host__ __device__ constexpr int spw_sm_states(int W) { return W <= 4 ? 1024 : 512; }
+__host__ __device__ constexpr int spw_sm_bytes(int W) { return spw_sm_states(W) * (4 * (8 * W + 1) + 3 * 16); }
+
+// Steps i0.. of a walk in one block while the tables are small (no launch per kernel of a step): the
+// bodies of the separate kernels with the block's barriers between them.  SM: tables, staging and indexes in
+// shared memory (stops, reason 1, before a step of more than min(limit, spw_sm_states(W)) / 2 states);
+// else in the scratch (reason 1 beyond limit / 2; reason 5 once 4 n <= back: the shared tables take it).
+// Reason 4: a step raised a flag and the walk is void.  state: [0] next step, [1] ring slot of its table,
+// [2] reason.
+//
+// Bound: the chain of dependent accesses of a step (state, staging claim, staged key, claim, index claim),
+// not bytes: in shared memory that chain is short, and what leaves the SM is the kept copies, the lookups
+// in a backward table and the step's counters.  A query of two-word states (2500 columns, K = 5) walks 59 ms,
+// 99 with all of it on the scratch; of three-word states with tables up to 10^4 (4001 columns, K = 5) 236, 279
+// (what stays on the scratch there, 512 to 2048 states a step, takes 189).  The next step's row is fetched during this one, its indexes are cleared beside the kept copy, and that copy is
+// written while the next step's states go in.
+template <int W, bool SM>
+__global__ void __launch_bounds__(SM ? SPW_SM_THREADS : SPW_SMALL_THREADS)
+    k_spw_walk_small(const __grid_constant__ SpwSmall S) {
+    extern __shared__ unsigned long long sm_wide[];
+    constexpr uint64_t N = (uint64_t)spw_sm_states(W);
+    const uint64_t cap = S.cap, M = SM ? N : cap, ME = SM ? N : 2 * cap;     // strides: tables, staging
+    const int r1 = (S.cur + 1) % 3;                      // the scratch's tables 0 and 1: ring slots cur and r1
+    // tables 0 and 1, staging 2, changed list 3
+    auto sH = [&](int t) {
+        if constexpr (SM) return sm_wide + (uint64_t)t * 2 * N;
+        else return t == 2 ? S.sg.H : S.ring[t ? r1 : S.cur].H;
+    };
+    auto sK = [&](int t) {
+        if constexpr (SM) return reinterpret_cast<uint64_t *>(sm_wide + 6 * N) + (uint64_t)t * W * N;
+        else return t == 3 ? S.ch.keys : t == 2 ? S.sg.keys : S.ring[t ? r1 : S.cur].keys;
+    };
+    auto sV = [&](int t) {
+        if constexpr (SM) return reinterpret_cast<uint8_t *>(sm_wide + 6 * N + 4 * W * N) + (uint64_t)t * N;
+        else return t == 3 ? S.ch.vals : t == 2 ? S.sg.vals : S.ring[t ? r1 : S.cur].vals;
+    };
     __shared__ WideStep P2[2];
     __shared__ WideBound B2[2];
     __shared__ uint64_t jt2[2][SPW_MAXW];
+    __shared__ int64_t F2[2][SPW_WALK_FIELDS];
+    __shared__ unsigned long long cs[2][8], jr[2], rs[8], used;
     const Lanes L = block_lanes();
     const unsigned tid = threadIdx.x;
     const bool lead = tid == 0;
     unsigned long long *abort = S.cnt + 8ull * (2 * (uint64_t)S.nsteps + 1) + 1, *state = abort + 1;
-    const uint64_t cap = S.cap;
-    auto load_row = [&](int i, int b) {                  // this block's copy of step i's parameters
-        const int64_t *f = S.steps + (size_t)SPW_WALK_FIELDS * i;
-        const uint64_t *wd = S.words + (size_t)5 * W * i;
-        const int ncls = f[WK_USEH] ? (int)f[WK_NCLS] : 0;
-        WideStep &P = P2[b];
-        WideBound &B = B2[b];
-        if (tid == 0) {
-            P.cap = (int)f[WK_CAP];
-            P.keep_below = (int)f[WK_KB];
-            P.w = (int)f[WK_W];
-            P.want_changed = f[WK_JOIN] != 0;
-            B.on = (int)f[WK_USEH];
-            B.ncls = ncls;
-            B.K = S.K;
-            B.extra = f[WK_EXTRA];
-        }
-        for (unsigned q = tid; q < (unsigned)W; q += blockDim.x) {
-            P.upd[q] = wd[q];
-            P.sel_mask[q] = wd[W + q];
-            P.sel_bits[q] = wd[2 * W + q];
-            B.tmask[q] = wd[3 * W + q];
-            jt2[b][q] = wd[4 * W + q];
-        }
-        for (unsigned c = tid; c < (unsigned)(ncls * W); c += blockDim.x)
-            B.mask[c / W][c % W] = S.masks[((size_t)i * S.maxc) * W + c];
-        for (unsigned c = tid; c < (unsigned)ncls; c += blockDim.x) B.w[c] = S.weights[(size_t)i * S.maxc + c];
+    const uint64_t limit = SM && N < S.limit ? N : S.limit;
+    auto load_row = [&](int i, int b) {
+        spw_load_row<W>(S, i, P2[b], B2[b], jt2[b]);
+        if (tid < SPW_WALK_FIELDS) F2[b][tid] = S.steps[(size_t)SPW_WALK_FIELDS * i + tid];
     };
-    int cur = S.cur, i = S.i0, reason = 0;
+    auto put = [&](unsigned long long *H, int lg, const uint64_t (&k)[W], unsigned long long word) {   // a new key
+        const uint32_t mask = (1u << lg) - 1u;
+        uint32_t t = spw_slot<W>(k, lg);
+        for (uint32_t probe = 0; probe <= mask; probe++) {
+            if (atomicCAS(H + t, SPW_EMPTY, word) == SPW_EMPTY) return;
+            t = (t + 1) & mask;
+        }
+    };
+    int cur = 0, i = S.i0, reason = 0;
     uint64_t n = 0;
     int lg_old = 0;
     {
         int noff, lgoff;
         const unsigned long long *pc = S.cnt + spw_prev_off(S.steps, i, noff, lgoff);
         n = spw_count(pc + noff, cap);
-        lg_old = (int)__ldcg(pc + lgoff);
+        lg_old = SM ? spw_lg_dev(n) : (int)__ldcg(pc + lgoff);
     }
-    if (i < S.nsteps && 2 * n <= S.limit) {
+    if (tid < 16) cs[tid / 8][tid % 8] = 0;
+    if (tid < 2) jr[tid] = SPW_EMPTY;
+    if (lead) used = __ldcg(abort - 1);
+    if (__ldcg(abort)) reason = 4;
+    if (i < S.nsteps && 2 * n <= limit) {
         load_row(i, i & 1);
         const int lgs = spw_lg_dev(2 * n);
-        spw_fill_body(L, S.sg.H, 1ull << lgs);
-        spw_fill_body(L, S.ring[(cur + 1) % 3].H, 1ull << lgs);
+        spw_fill_body(L, sH(1), 1ull << lgs);
+        spw_fill_body(L, sH(2), 1ull << lgs);
+        if (SM) {                                        // the table before step i0, re-indexed
+            spw_fill_body(L, sH(0), 1ull << lg_old);
+            __syncthreads();
+        }
+        for (uint64_t q = tid; SM && q < n; q += blockDim.x) {
+            uint64_t k[W];
+            spw_load<W>(S.ring[S.cur].keys, cap, q, k);
+            const uint8_t v = S.ring[S.cur].vals[q];
+#pragma unroll
+            for (int w = 0; w < W; w++) sK(0)[(uint64_t)w * N + q] = k[w];
+            sV(0)[q] = v;
+            put(sH(0), lg_old, k, ((unsigned long long)v << 56) | q);
+        }
     }
-    if (__ldcg(abort)) reason = 4;
     __syncthreads();
     for (; i < S.nsteps && !reason; i++) {
-        if (2 * n > S.limit) { reason = 1; break; }
-        const WideStep &P = P2[i & 1];
-        const WideBound &B = B2[i & 1];
-        const int64_t *f = S.steps + (size_t)SPW_WALK_FIELDS * i;
+        if (2 * n > limit) { reason = 1; break; }
+        if (!SM && i > S.i0 && 4 * n <= S.back) { reason = 5; break; }
+        const int b = i & 1;
+        const WideStep &P = P2[b];
+        const WideBound &B = B2[b];
+        const int64_t *f = F2[b];
         const unsigned long long *jH = reinterpret_cast<const unsigned long long *>((uintptr_t)f[WK_JH]);
         const uint64_t *jk = reinterpret_cast<const uint64_t *>((uintptr_t)f[WK_JKEYS]);
         const bool join = f[WK_JOIN] && jH && jk;
-        unsigned long long *c = S.cnt + 8ull * (i + 1), *rec = S.cnt + 8ull * (S.nsteps + 1 + i);
-        const int lgs = spw_lg_dev(2 * n);
-        if (lead) c[3] = (unsigned long long)lgs;
-        const int out = (cur + 1) % 3;
-        spw_emit_body<W, true>(L, S.ring[cur].keys, S.ring[cur].vals, n, cap, S.sg.keys, S.sg.vals, 2 * cap, S.sg.H, lgs, P, B,
-                         c);
-        if (i + 1 < S.nsteps) load_row(i + 1, (i + 1) & 1);
+        unsigned long long *c = cs[b], *gc = S.cnt + 8ull * (i + 1), *rec = S.cnt + 8ull * (S.nsteps + 1 + i);
+        const int lgs = spw_lg_dev(2 * n), out = cur ^ 1;
+        if (tid < 8) cs[b ^ 1][tid] = 0;
+        if (lead) {
+            jr[b ^ 1] = SPW_EMPTY;
+            c[3] = (unsigned long long)lgs;
+        }
+        spw_emit_body<W, true, SM>(L, sK(cur), sV(cur), n, M, sK(2), sV(2), ME, sH(2), lgs, P, B, c);
+        if (i + 1 < S.nsteps) load_row(i + 1, b ^ 1);
         __syncthreads();
-        spw_compact_body<W>(L, S.sg.H, 1ull << lgs, S.sg.keys, 2 * cap, S.ring[out].keys, S.ring[out].vals, cap,
-                            S.ring[out].H, lgs, S.ch.keys, S.ch.vals, cap, S.ring[cur].H, lg_old, S.ring[cur].keys,
-                            cap, P, c);
+        spw_compact_body<W, SM>(L, sH(2), 1ull << lgs, sK(2), ME, sK(out), sV(out), M, sH(out), lgs, sK(3), sV(3), M,
+                                sH(cur), lg_old, sK(cur), M, P, c);
         __syncthreads();
-        if (__ldcg(c + 2) & 7ull) { reason = 4; break; }
-        const uint64_t nout = spw_count(c, cap);
+        if (c[2] & 7ull) { reason = 4; if (tid < 8) gc[tid] = c[tid]; break; }
+        const uint64_t nout = c[0];
         if (join)
-            spw_join_body<W>(L, S.ch.keys, S.ch.vals, spw_count(c + 1, cap), cap, jH, (int)f[WK_JLG], jk,
-                             (uint64_t)f[WK_JSTRIDE], jt2[i & 1], S.res + i, 0);
+            spw_join_body<W>(L, sK(3), sV(3), c[1], M, jH, (int)f[WK_JLG], jk, (uint64_t)f[WK_JSTRIDE], jt2[b],
+                             &jr[b], 0);
         int now = out, lgn = lgs;
         uint64_t nnow = nout;
         if (f[WK_TRUNC] >= 0) {
             // the cap drops at this cut: the whole table before the drop is joined too
             if (join)
-                spw_join_body<W>(L, S.ring[out].keys, S.ring[out].vals, nout, cap, jH, (int)f[WK_JLG], jk,
-                                 (uint64_t)f[WK_JSTRIDE], jt2[i & 1], S.res + i, SPW_TAG);
-            now = (out + 1) % 3;
+                spw_join_body<W>(L, sK(out), sV(out), nout, M, jH, (int)f[WK_JLG], jk, (uint64_t)f[WK_JSTRIDE],
+                                 jt2[b], &jr[b], SPW_TAG);
+            now = cur;
             lgn = spw_lg_dev(nout);
             if (lead) c[5] = (unsigned long long)lgn;
-            spw_fill_body(L, S.ring[now].H, 1ull << lgn);
+            spw_fill_body(L, sH(now), 1ull << lgn);
             __syncthreads();
-            spw_filter_body<W>(L, S.ring[out].keys, S.ring[out].vals, nout, cap, (int)f[WK_TRUNC], S.ring[now].keys,
-                               S.ring[now].vals, cap, S.ring[now].H, lgn, c + 4);
+            spw_filter_body<W>(L, sK(out), sV(out), nout, M, (int)f[WK_TRUNC], sK(now), sV(now), M, sH(now), lgn, c + 4);
             __syncthreads();
-            if (__ldcg(c + 6) & 7ull) { reason = 4; break; }
-            nnow = spw_count(c + 4, cap);
+            if (c[6] & 7ull) { reason = 4; if (tid < 8) gc[tid] = c[tid]; break; }
+            nnow = c[4];
         }
-        if (f[WK_KEEP] && lead) spw_keep_place(nnow, W, (int)f[WK_KEEP], rec, abort - 1, S.arena ? S.arena_bytes : 0);
+        if (lead) {
+            for (int q = 0; q < 8; q++) rs[q] = 0;
+            if (f[WK_KEEP]) {
+                spw_keep_place(nnow, W, (int)f[WK_KEEP], rs, &used, S.arena ? S.arena_bytes : 0);
+                rec[0] = (rs[2] & 24ull) ? 0 : nnow;
+                for (int q = 1; q < 5; q++) rec[q] = rs[q];
+            }
+        }
         __syncthreads();
-        const bool keep = f[WK_KEEP] && !(__ldcg(rec + 2) & 24ull);
-        if (join && lead)
-            spw_capture_one<W>(S.res + i, S.ch.keys, S.ch.vals, S.ring[out].keys, S.ring[out].vals, cap,
-                               S.resk + (size_t)i * W, S.resv + i);
-        if (keep) spw_fill_body(L, spw_keep_index(S.arena, rec, W), 1ull << __ldcg(rec + 3));
+        const bool keep = f[WK_KEEP] && !(rs[2] & 24ull);
+        const uint64_t ks = rs[4];
+        uint8_t *kp = S.arena + rs[1];
+        unsigned long long *kH =
+            reinterpret_cast<unsigned long long *>(kp + (uint64_t)W * ks * 8 + (ks + 255) / 256 * 256);
+        const int lgk = (int)rs[3];
+        if (tid < 8) gc[tid] = c[tid];
+        if (join && lead && jr[b] != SPW_EMPTY) {        // the state behind the join's result, for the host
+            const unsigned long long r = jr[b];
+            const uint64_t q = r & (SPW_TAG - 1);
+            const int t = (r & SPW_TAG) ? out : 3;
+            S.res[i] = r;
+#pragma unroll
+            for (int w = 0; w < W; w++) S.resk[(size_t)i * W + w] = sK(t)[(uint64_t)w * M + q];
+            S.resv[i] = sV(t)[q];
+        }
+        if (keep) spw_fill_body(L, kH, 1ull << lgk);
         cur = now;
         n = nnow;
         lg_old = lgn;
-        if (i + 1 < S.nsteps && 2 * n <= S.limit) {      // the next step's staging and new index
+        if (i + 1 < S.nsteps && 2 * n <= limit) {        // the next step's staging and new index
             const int lgx = spw_lg_dev(2 * n);
-            spw_fill_body(L, S.sg.H, 1ull << lgx);
-            spw_fill_body(L, S.ring[(cur + 1) % 3].H, 1ull << lgx);
+            spw_fill_body(L, sH(2), 1ull << lgx);
+            spw_fill_body(L, sH(cur ^ 1), 1ull << lgx);
         }
         __syncthreads();
-        if (keep) spw_keep_body<W>(L, S.ring[cur].keys, S.ring[cur].vals, n, cap, S.arena, rec);
+        if (keep)
+            for (uint64_t q = tid; q < n; q += blockDim.x) {
+                uint64_t k[W];
+                spw_load<W>(sK(cur), M, q, k);
+                const uint8_t v = sV(cur)[q];
+#pragma unroll
+                for (int w = 0; w < W; w++) reinterpret_cast<uint64_t *>(kp)[(uint64_t)w * ks + q] = k[w];
+                kp[(uint64_t)W * ks * 8 + q] = v;
+                put(kH, lgk, k, ((unsigned long long)v << 56) | q);
+            }
+    }
+    // the current table to a ring slot that it did not come from
+    const int gs = (S.cur + 1) % 3;
+    const bool moved = i > S.i0 && reason != 4;
+    if (SM && moved) {
+        for (uint64_t q = tid; q < n; q += blockDim.x) {
+#pragma unroll
+            for (int w = 0; w < W; w++) S.ring[gs].keys[(uint64_t)w * cap + q] = sK(cur)[(uint64_t)w * N + q];
+            S.ring[gs].vals[q] = sV(cur)[q];
+        }
+        for (uint64_t q = tid; q < (1ull << lg_old); q += blockDim.x) S.ring[gs].H[q] = sH(cur)[q];
     }
     if (lead) {
+        abort[-1] = used;
         if (reason == 4) *abort = 1;
         state[0] = (unsigned long long)i;
-        state[1] = (unsigned long long)cur;
+        state[1] = (unsigned long long)(!moved ? S.cur : SM ? gs : cur ? r1 : S.cur);
         state[2] = (unsigned long long)reason;
     }
 }
@@ -906,6 +1021,9 @@ static int spw_walk_w(int nsteps, const int64_t *steps, const uint64_t *words, c
         const int64_t *f = steps + (size_t)SPW_WALK_FIELDS * q;
         if (f[WK_CAP] > 254 || f[WK_W] < 1 || f[WK_W] > 254) limit = std::min<uint64_t>(limit, 512);
     }
+    e = cuda_check(cudaFuncSetAttribute(k_spw_walk_small<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        spw_sm_bytes(W)), "wide walk shared memory");
+    if (e) return e;
     uint64_t host_n = n0;             // the table size before step i, when known on the host
     int cur = 0, i = 0;
     while (i < nsteps) {
@@ -931,13 +1049,23 @@ static int spw_walk_w(int nsteps, const int64_t *steps, const uint64_t *words, c
             S.resk = resk;
             S.resv = resv;
             S.arena = arena;
-            k_spw_walk_small<W><<<1, SPW_SMALL_THREADS, 0, st>>>(S);
-            e = cuda_check(cudaGetLastError(), "small wide walk");
-            if (!e) e = cuda_check(cudaMemcpyAsync(hb, sstate, 24, cudaMemcpyDeviceToHost, st), "walk state");
-            if (!e) e = cuda_check(cudaStreamSynchronize(st), "walk sync");
-            if (e) return e;
-            i = (int)hb[0];
-            cur = (int)hb[1];
+            S.back = limit < (uint64_t)spw_sm_states(W) ? limit : (uint64_t)spw_sm_states(W);
+            bool shared = 2 * host_n <= S.back;
+            while (true) {
+                S.i0 = i;
+                S.cur = cur;
+                if (shared) k_spw_walk_small<W, true><<<1, SPW_SM_THREADS, spw_sm_bytes(W), st>>>(S);
+                else k_spw_walk_small<W, false><<<1, SPW_SMALL_THREADS, 0, st>>>(S);
+                e = cuda_check(cudaGetLastError(), "small wide walk");
+                if (!e) e = cuda_check(cudaMemcpyAsync(hb, sstate, 24, cudaMemcpyDeviceToHost, st), "walk state");
+                if (!e) e = cuda_check(cudaStreamSynchronize(st), "walk sync");
+                if (e) return e;
+                i = (int)hb[0];
+                cur = (int)hb[1];
+                // beyond the shared tables the L2 ones go on, and hand back what has shrunk
+                if (shared ? (hb[2] != 1 || limit <= S.back) : hb[2] != 5) break;
+                shared = !shared;
+            }
             if (hb[2] == 4) break;    // a flag: the walk is void, the host reads why at the end
             host_n = ~0ull >> 3;      // beyond the limit until read again
             if (i >= nsteps) break;
