@@ -96,3 +96,14 @@ def test_batched_passes_match_single(lib, seed):
     got = DenseBatch(plans).run()
     for pl, v in zip(plans, got):
         assert v == (kernel.run_plan(pl)[0] if pl.feasible else None)
+
+
+@pytest.mark.parametrize("every,gran", [(1, False), (3, False), (4, True), (16, True)])
+def test_checkpoints_every_few_ops_take_the_other_forms(every, gran):
+    """A granule pass between checkpoints an op or two apart would hold one column."""
+    from tropidist_gb300 import kernel
+    p = synth.banded(120, 300, 18, 3, 1, seed=3)
+    plan = trellis.build_plan(p.h, p.l, 1, list(range(300)), p.nrows)
+    cp = kernel.CompiledPlan(plan, "u8", list(range(every, len(plan.ops), every)))
+    assert (4 in cp.segments()[:, 0]) == gran
+    cp.free()

@@ -755,7 +755,9 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
     const int DMAX = eb == 1 ? g_dmax8 : g_dmax16;
     const int SWB = eb == 1 ? g_sweep_bits8 : g_sweep_bits16;
     const bool relayout = eb == 1 && g_relayout;
-    const bool gran = use_gran(eb);
+    // a table kept after every op or two (a leaf of the witness traceback) leaves a granule pass one column:
+    // the other forms need no reordering there (26-bit witness: 156 ms, 209 with granule passes in the leaves)
+    const bool gran = use_gran(eb) && nops >= 4 * nckpt;
     P.eb = eb;
     P.peak_bits = peak;
     P.nops = nops;
