@@ -701,9 +701,9 @@ def main():
                 else:
                     cp.execute(a, b)
             else:
-                out = (ctypes.c_double * 12)()
-                _lib.check(L.tg_dense_execute_timed(cp.handle, a.data_ptr(), b.data_ptr(), st.cuda_stream, out, 12))
-                for k in range(12):
+                out = (ctypes.c_double * 15)()
+                _lib.check(L.tg_dense_execute_timed(cp.handle, a.data_ptr(), b.data_ptr(), st.cuda_stream, out, 15))
+                for k in range(15):
                     timed[k] += out[k]
             vals.append(cp)
         if timed is None:
@@ -721,7 +721,7 @@ def main():
         os.environ.get("CUDA_VISIBLE_DEVICES", "").split(",")[0].isdigit() else str(local)
     clocks = Clocks(gpu_index)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    acc = [0.0] * 12
+    acc = [0.0] * 15
     e0.record(st)
     for _ in range(args.steps):
         step()
@@ -767,8 +767,8 @@ def main():
         e2e_value = None
 
     peak_gbs, peak_kind = measured_peak()
-    # the dominant kernel by GPU time: coset-streaming passes or fused tile passes
-    kinds = {"k_fused_pass_u8": 1, "k_stream_pass_u8": 3}
+    # the dominant kernel by GPU time: granule, coset-streaming or fused tile passes
+    kinds = {"k_fused_pass_u8": 1, "k_stream_pass_u8": 3, "k_gran_pass": 4}
     kname = max(kinds, key=lambda k: acc[3 * kinds[k] + 1])
     ki = kinds[kname]
     n_fp, ms_fp, bytes_fp = acc[3 * ki], acc[3 * ki + 1], acc[3 * ki + 2]
@@ -795,8 +795,9 @@ def main():
             "vs_baseline": None, "dtype": "u8", "data": "synthetic (seeded banded problem)",
             "config": config(args, plans, dists),
             "parallelism": "replicas (one instance per rank)" if world > 1 else "1 GPU",
-            "schedule": {"streams": 2, "fused_passes_per_step": int((acc[3] + acc[9]) / args.steps),
+            "schedule": {"streams": 2, "fused_passes_per_step": int((acc[3] + acc[9] + acc[12]) / args.steps),
                          "streaming_passes_per_step": int(acc[9] / args.steps),
+                         "granule_passes_per_step": int(acc[12] / args.steps),
                          "segments_per_step": sum(cp.nsegs for cp in cps)},
             "parity": {"reference_fixture": dist_string(gold) if gold else None,
                        "equal": (dists == gold) if gold else None},

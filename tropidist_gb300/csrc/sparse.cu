@@ -458,11 +458,11 @@ __host__ __device__ static int lg_tiny(uint64_t m) {
 
 // ---- tables that fit shared memory: the same steps with the old table, the new one and the changed list
 // there, so that index probes and claims are shared-memory atomics: from the global scratch one SM's
-// random L2 atomics bound the step.  It takes tables of at most SPW_TINY_N / 2
-// states and stops (reason 1) when a step would need more.  The next step's row is fetched during this
-// one.  A kept table is a plain copy of its states and of the working index (load 1/4 to 1/2), unless
-// that index is more than twice what the table needs.  The truncated table of a cut takes the old
-// table's place, free by then.  The table it ends with is written to a global scratch slot.
+// random L2 atomics bound the step.  It takes tables of at most SPW_TINY_N / 2 states and stops (reason 1)
+// when a step would need more.  The next step's row is fetched during this one.  A kept table is a plain
+// copy of its states and of the working index (load 1/4 to 1/2), unless that index is more than twice what
+// the table needs.  The truncated table of a cut takes the old table's place, free by then.  The table it
+// ends with is written to a global scratch slot.
 #define SPW_TINY_N 4096
 #define SPW_TINY_LG 13
 #define SPW_TINY_THREADS 1024

@@ -657,9 +657,9 @@ __host__ __device__ constexpr int spw_sm_bytes(int W) { return spw_sm_states(W) 
 // Bound: the chain of dependent accesses of a step (state, staging claim, staged key, claim, index claim),
 // not bytes: in shared memory that chain is short, and what leaves the SM is the kept copies, the lookups
 // in a backward table and the step's counters.  A query of two-word states (2500 columns, K = 5) walks 59 ms,
-// 99 with all of it on the scratch; of three-word states with tables up to 10^4 (4001 columns, K = 5) 236, 279
-// (what stays on the scratch there, 512 to 2048 states a step, takes 189).  The next step's row is fetched during this one, its indexes are cleared beside the kept copy, and that copy is
-// written while the next step's states go in.
+// 99 with all of it on the scratch; one of three-word states with tables beyond it (4001 columns, K = 5)
+// 236 ms, 279 (189 of them on the scratch).  The next step's row is fetched during this one, its indexes
+// are cleared beside the kept copy, and that copy is written while the next step's states go in.
 template <int W, bool SM>
 __global__ void __launch_bounds__(SM ? SPW_SM_THREADS : SPW_SMALL_THREADS)
     k_spw_walk_small(const __grid_constant__ SpwSmall S) {
