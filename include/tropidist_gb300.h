@@ -114,6 +114,10 @@ int tg_dense_witness_small(const int64_t *ops, int64_t n, int eb, void *tables, 
 /* Runs a scheduled plan on HOST buffers with the launch parameters and index arithmetic of the
  * kernels; for checking the scheduler on a machine without a GPU.  Not an evaluator. */
 int tg_debug_emulate_dense(void *plan, void *host_a, void *host_b, void **ckpt_host);
+/* Address maps of segment `seg`, a granule pass (kind 4), for the same purpose: input and output offsets,
+ * in 4-byte granules, of the pass's coset-number bits and register slots (in, out: HOST uint32 [40]; n[0]
+ * and n[1] of them).  The pass reads and writes every granule once when each list is independent. */
+int tg_debug_gran_maps(void *plan, int64_t seg, uint32_t *in, uint32_t *out, int *n);
 
 /* ---------------------------------------------------------------- sparse Rank DP (device tables)
  * A table: n packed states key | value << 56 (key = row-slot parities, <= 56 slots; value 0..254),

@@ -103,6 +103,7 @@ def _declare(L):
         "tg_dense_set_tuning": (ci, [ci, ci, ci, ci]),
         "tg_dense_set_stream_span": (ci, [ci, ci]),
         "tg_debug_emulate_dense": (ci, [vp, vp, vp, vp]),
+        "tg_debug_gran_maps": (ci, [vp, i64, vp, vp, vp]),
     }
     from . import _sigs_extra
     sig.update(_sigs_extra.SIGNATURES)

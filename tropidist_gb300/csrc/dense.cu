@@ -2116,6 +2116,24 @@ int tg_debug_emulate_dense(void *plan, void *host_a, void *host_b, void **ckpt_h
     return TG_OK;
 }
 
+int tg_debug_gran_maps(void *plan, int64_t seg, uint32_t *in, uint32_t *out, int *n) {
+    if (!plan || !in || !out || !n) return set_error(TG_ERR_ARG, "null argument");
+    const DensePlan &P = *static_cast<DensePlan *>(plan);
+    if (seg < 0 || seg >= (int64_t)P.segs.size() || P.segs[seg].kind != 4) return set_error(TG_ERR_ARG, "not a granule pass");
+    const GranParams &g = P.segs[seg].gp;
+    n[0] = n[1] = 0;
+    for (int b = 0; b < g.nk; b++) {
+        const uint2 o = b < 8 ? g.klow[b] : g.khigh[(b - 8) / 4][1 << ((b - 8) & 3)];
+        in[n[0]++] = o.x;
+        out[n[1]++] = o.y;
+    }
+    for (int s = 0; s < GP_SLOTS; s++) {
+        if (s < g.nload) in[n[0]++] = g.xin[1 << s] ^ g.xin[0];
+        if ((g.live_out >> (1 << s)) & 1u) out[n[1]++] = g.mout[1 << s].x ^ g.mout[0].x;
+    }
+    return TG_OK;
+}
+
 int tg_dense_run_noalloc(const int64_t *ops, int64_t nops, uint8_t *table_dev, uint64_t table_entries,
                          uint32_t *value, void *stream) {
     if (!value || (nops > 0 && !ops) || nops < 0) return set_error(TG_ERR_ARG, "bad op stream or result pointer");

@@ -56,7 +56,8 @@ struct GranParams {
     uint64_t ncosets;                // 2^nk
     int nk, nload, nops, pad;        // coset-number bits, slots loaded (0 .. nload - 1)
     uint32_t live_out;               // members stored (bit z)
-    uint32_t fin, fout;              // constant parts of the offsets (granules)
+    uint32_t fin, fout;              // constant parts of the offsets (granules; every offset is 32-bit, so
+                                     // tables hold at most 2^GP_MAXBITS granules)
     uint32_t smask0, smask1;         // coset-number bits flipping in-granule bit 0 / 1 of the output
     GranOp ops[GP_MAXOPS];
     uint32_t xin[GP_MEMBERS];        // member z: input offset

@@ -6,6 +6,7 @@
 namespace tg {
 
 #define GP_MINW 9            // narrowest table of a pass (input and output)
+#define GP_MAXBITS 32        // widest, in granules: the kernel's offsets are 32-bit granule numbers
 #define GP_EVICT_OPS 40      // an in-granule row that closes within this many ops leaves the granule
 
 // value of a row as a parity of register slots, coset-number bits and a constant
@@ -26,8 +27,9 @@ struct GranCol {
 
 // Builds the pass that starts at op i0 on the table with rows `phys` (canonical order `canon`);
 // ops before `limit` may be taken.  Returns the first op not taken, with canon / phys brought to the
-// pass's output (i0 when only rows changed places); -1 when the form does not apply; -2 on an
-// internal inconsistency.  nupd: updates taken.
+// pass's output (i0 when only rows changed places); -1 when the form does not apply (tables of more than
+// 2^GP_MAXBITS granules, read or written, take the other forms); -2 on an internal
+// inconsistency.  nupd: updates taken.
 //
 // Local row numbers: input rows by physical position, then the rows opened in the pass.  With column
 // m's use as variable z_m, a state is s_base + sum z_m h_m.  A column that opens a row has no free
@@ -36,7 +38,7 @@ struct GranCol {
 static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, int64_t i0, int64_t limit, int eb,
                           std::vector<int> &canon, std::vector<int> &phys, GranParams &gp, int &nupd) {
     const int G = eb == 1 ? 2 : 1, w_in = (int)phys.size();
-    if (w_in < GP_MINW || w_in > 40) return -1;
+    if (w_in < GP_MINW || w_in > GP_MAXBITS + G) return -1;
     static thread_local std::vector<int> where;          // row -> local number
     if (where.size() < RI.uses.size()) where.resize(RI.uses.size());
     int rowid[64];
@@ -119,7 +121,8 @@ static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, in
             if (((C.h >> l) & 1ull) && l != C.r) { C.c = l; C.t = (int)hops[kn].b; kn++; }
         }
         C.type = open ? (C.c >= 0 ? GC_A : GC_O) : (C.c >= 0 ? GC_C : GC_N);
-        if (nc_rows + (open ? 1 : 0) - (C.c >= 0 ? 1 : 0) < GP_MINW) break;
+        const int w_next = nc_rows + (open ? 1 : 0) - (C.c >= 0 ? 1 : 0);
+        if (w_next < GP_MINW || w_next > GP_MAXBITS + G) break;
         int L2 = L, M2 = M;
         uint64_t red = 0;
         if (!open) {
