@@ -64,6 +64,10 @@ int tg_dense_plan_info(void *plan, int64_t *info, int ninfo);
  * an in-chunk part), store mode */
 int tg_dense_plan_segments(void *plan, int64_t *out, int64_t maxseg);
 void tg_dense_plan_free(void *plan);
+/* buf_a, buf_b: DEVICE, 2^peak_bits entries each.  16-byte aligned buffers suit every plan; a plan of
+ * sweeps alone runs on any buffer of whole entries, one of sweeps and granule passes on 4-byte aligned ones;
+ * TG_ERR_ARG, and nothing launched, where a pass needs more (the same for every call below that runs a
+ * plan; tg_dense_plan_execute has the segments before that pass queued by then). */
 int tg_dense_execute(void *plan, void *buf_a, void *buf_b, void **ckpt_bufs, void *stream);
 int tg_dense_result(void *plan, void *buf_a, void *buf_b, uint32_t *value, void *stream);
 /* execute with a CUDA event pair around every launch (on `stream`), waits for the end; out[15]:

@@ -1187,6 +1187,22 @@ static int ensure_events(size_t n) {
     return TG_OK;
 }
 
+// Alignment that a segment's kernel needs of both tables: an entry in sweeps (and in a select that goes entry
+// by entry), a granule in granule passes, a 16-byte chunk in the others.
+static int check_aligned(const Seg &S, int eb, const void *a, const void *b) {
+    const bool scalar = S.kind == 0 || (S.kind == 2 && S.op_code == 2 && S.op_a < (eb == 1 ? 4u : 3u));
+    const uintptr_t need = scalar ? (uintptr_t)eb : S.kind == 4 ? 4 : 16;
+    if (((uintptr_t)a | (uintptr_t)b) % need)
+        return set_error(TG_ERR_ARG, "table buffer not aligned for the plan's passes (16 bytes suit every plan)");
+    return TG_OK;
+}
+
+static int check_aligned(const DensePlan &P, const void *a, const void *b) {
+    for (const Seg &S : P.segs)
+        if (check_aligned(S, P.eb, a, b)) return TG_ERR_ARG;
+    return TG_OK;
+}
+
 template <typename E>
 static int launch_seg(const Seg &S, E *const bufs[2], int &cur, void **ckpt_bufs, cudaStream_t st, size_t si,
                       bool timed) {
@@ -1269,6 +1285,8 @@ struct SegLauncher {
 
 static int launch_hook(const Seg &S, void *ctx) {
     SegLauncher &Lr = *static_cast<SegLauncher *>(ctx);
+    const int e = check_aligned(S, Lr.eb, Lr.bufs[0], Lr.bufs[1]);
+    if (e) return e;
     if (Lr.eb == 1) {
         uint8_t *const b[2] = {static_cast<uint8_t *>(Lr.bufs[0]), static_cast<uint8_t *>(Lr.bufs[1])};
         return launch_seg<uint8_t>(S, b, Lr.cur, nullptr, Lr.st, 0, false);
@@ -2041,8 +2059,9 @@ int tg_dense_execute(void *plan, void *buf_a, void *buf_b, void **ckpt_bufs, voi
     if (!plan || !buf_a || !buf_b) return set_error(TG_ERR_ARG, "null plan or buffer");
     const DensePlan &P = *static_cast<DensePlan *>(plan);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    int e = check_aligned(P, buf_a, buf_b);
+    if (e) return e;
     // the start table {0: 0} in buffer a (a plan from a given table finds it there)
-    int e = TG_OK;
     if (P.w_start == 0) e = cuda_check(cudaMemsetAsync(buf_a, 0, P.eb, st), "init");
     if (e) return e;
     if (P.nops == 0) return TG_OK;
@@ -2056,7 +2075,8 @@ int tg_dense_execute_timed(void *plan, void *buf_a, void *buf_b, void *stream, d
     if (!plan || !buf_a || !buf_b || !out) return set_error(TG_ERR_ARG, "null argument");
     const DensePlan &P = *static_cast<DensePlan *>(plan);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int e = cuda_check(cudaMemsetAsync(buf_a, 0, P.eb, st), "init");
+    int e = check_aligned(P, buf_a, buf_b);
+    if (!e) e = cuda_check(cudaMemsetAsync(buf_a, 0, P.eb, st), "init");
     if (e) return e;
     if (P.eb == 1) e = launch_plan<uint8_t>(P, (uint8_t *)buf_a, (uint8_t *)buf_b, nullptr, st, true);
     else e = launch_plan<uint16_t>(P, (uint16_t *)buf_a, (uint16_t *)buf_b, nullptr, st, true);
@@ -2144,6 +2164,7 @@ int tg_dense_run_noalloc(const int64_t *ops, int64_t nops, uint8_t *table_dev, u
     if (P.peak_bits > TG_NOALLOC_MAX_BITS)
         return set_error(TG_ERR_TOO_BIG, "plan wider than the 2^22-entry scratch of tg_dense_run_noalloc");
     if (table_entries < (1ull << P.peak_bits)) return set_error(TG_ERR_ARG, "table buffer smaller than 2^peak_bits");
+    if ((e = check_aligned(P, table_dev, table_dev))) return e;
     uint8_t *scratch = nullptr;
     e = noalloc_scratch(&scratch);
     if (e) return e;

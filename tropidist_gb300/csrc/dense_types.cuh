@@ -78,7 +78,9 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P, const E *__rest
     E *S = T + (1u << P.max_bits);
     int bits = P.w_in;
     uint32_t n = 1u << bits;
-    if (P.has_in && bits >= CB) {
+    // buffers that are not 16-byte aligned go entry by entry (a plan of sweeps alone runs on any buffer)
+    const bool in16 = (reinterpret_cast<uintptr_t>(in) & 15u) == 0, out16 = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    if (P.has_in && bits >= CB && in16) {
         // 16-byte loads in physical order, entries to their canonical places
         for (uint32_t c = threadIdx.x; c < (n >> CB); c += blockDim.x) {
             const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(in) + c);
@@ -126,7 +128,7 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P, const E *__rest
         }
         __syncthreads();
     }
-    if (bits >= CB) {
+    if (bits >= CB && out16) {
         for (uint32_t c = threadIdx.x; c < (n >> CB); c += blockDim.x) {
             uint4 v;
             E *e = reinterpret_cast<E *>(&v);
