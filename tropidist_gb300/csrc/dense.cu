@@ -938,7 +938,7 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
                 uint32_t m = 0;
                 for (int r : upd[u].first) m |= 1u << index_of(local, r);
                 pp.upd_mask[u] = m;
-                pp.upd_w[u] = (uint8_t)upd[u].second;
+                pp.upd_w[u] = (uint16_t)upd[u].second;
             }
             if (eb == 1) {
                 build_groups(pp, selmask);
@@ -1000,10 +1000,10 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
                     sp.ops[sp.nops++] = 0u;
                     w++;
                 } else if (o.code == 1) {
-                    sp.ops[sp.nops++] = (1u << 30) | ((uint32_t)o.b << 20) | (uint32_t)o.a;
+                    sp.ops[sp.nops++] = SW_UPDATE | ((uint32_t)o.b << sw_wshift(eb)) | (uint32_t)o.a;
                     P.n_updates++;
                 } else {
-                    sp.ops[sp.nops++] = (2u << 30) | ((uint32_t)o.b << 6) | (uint32_t)o.a;
+                    sp.ops[sp.nops++] = SW_SELECT | ((uint32_t)o.b << 6) | (uint32_t)o.a;
                     w--;
                 }
                 apply_canon(j, canon);
@@ -1488,12 +1488,12 @@ static void emulate_plan(const DensePlan &P, E *a, E *b, void **ckpt) {
             if (S.sp.has_in)
                 for (size_t x = 0; x < T.size(); x++) T[canon_index(x, S.sp.in_pos, S.sp.w_in)] = src[x];
             for (int i = 0; i < S.sp.nops; i++) {
-                uint32_t op = S.sp.ops[i], code = op >> 30;
+                uint32_t op = S.sp.ops[i];
                 size_t n = T.size();
-                if (code == 0) {
+                if (!(op & (SW_UPDATE | SW_SELECT))) {
                     T.resize(2 * n, (E)INF);
-                } else if (code == 1) {
-                    uint32_t m = op & 0xFFFFFu, w = (op >> 20) & 0xFFu;
+                } else if (op & SW_UPDATE) {
+                    uint32_t m = sw_mask(op, sizeof(E)), w = sw_weight(op, sizeof(E));
                     int hb = 31 - __builtin_clz(m);
                     for (uint32_t s = 0; s < n; s++) {
                         if ((s >> hb) & 1) continue;

@@ -49,9 +49,17 @@ __device__ __forceinline__ void smem_update(E *T, int bits, uint32_t m, uint32_t
 }
 
 // ------------------------------------------------------------------ single-CTA sweep (narrow tables)
-// Op words: bits 30-31 code (0 expand, 1 update, 2 select); update: mask in bits 0-19, weight in
-// bits 20-27; select: pos in bits 0-5, target in bit 6.
+// Op words: bit 31 set: update, the mask in the bits below sw_wshift and the weight from there (uint8: 20
+// bits and 8, uint16: tables of at most 15 bits, 15 bits and the whole 16-bit weight); else bit 30 set:
+// select, pos in bits 0-5, target in bit 6; else expand.
 #define SW_MAXOPS 900
+#define SW_UPDATE (1u << 31)
+#define SW_SELECT (1u << 30)
+__host__ __device__ constexpr int sw_wshift(int eb) { return eb == 1 ? 20 : 15; }
+__host__ __device__ __forceinline__ uint32_t sw_mask(uint32_t op, int eb) { return op & ((1u << sw_wshift(eb)) - 1u); }
+__host__ __device__ __forceinline__ uint32_t sw_weight(uint32_t op, int eb) {
+    return (op >> sw_wshift(eb)) & (eb == 1 ? 0xFFu : 0xFFFFu);
+}
 struct SweepParams {
     int nops;
     int w_in;             // width of the input table (0: start from {0: 0})
@@ -102,13 +110,12 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P, const E *__rest
     __syncthreads();
     for (int i = 0; i < P.nops; i++) {
         const uint32_t op = P.ops[i];
-        const uint32_t code = op >> 30;
-        if (code == 0) {
+        if (op & SW_UPDATE) {
+            smem_update<E>(T, bits, sw_mask(op, sizeof(E)), sw_weight(op, sizeof(E)));
+        } else if (!(op & SW_SELECT)) {
             for (uint32_t s = threadIdx.x; s < n; s += blockDim.x) T[n + s] = (E)Entry<E>::INF;
             bits++;
             n <<= 1;
-        } else if (code == 1) {
-            smem_update<E>(T, bits, op & 0xFFFFFu, (op >> 20) & 0xFFu);
         } else {
             const int pos = op & 63;
             const uint32_t tgt = (op >> 6) & 1u;
@@ -161,7 +168,7 @@ struct PassParams {
     uint32_t cmp_smem[FP_MAXD];        // smem entry weight of compacted local bit j
     uint64_t outer_in[FP_MAXOUTER], outer_out[FP_MAXOUTER];
     uint32_t upd_mask[FP_MAXU];
-    uint8_t upd_w[FP_MAXU];
+    uint16_t upd_w[FP_MAXU];           // uint16 tables: weights up to 65534
     uint16_t pat[16];                  // smem index of the low compacted entries (generic store)
     // uint8 register-group form of the same updates (k_fused_pass_u8)
     int use_groups, ngroups;
