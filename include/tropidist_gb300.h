@@ -264,7 +264,9 @@ void tab_build(void *t, int n, const uint64_t *zh, const uint64_t *zl, const uin
 /* ---------------------------------------------------------------- batched dense Rank DP
  * Many plans (op streams ops[offsets[i]..offsets[i+1]), uint8) in one persistent launch fed from a
  * device work queue.  No counterpart in the reference, which runs one plan at a time
- * (cdist/auto.py:111-122).  info: arena bytes, jobs, units, plans.  values: HOST uint32[nplans]. */
+ * (cdist/auto.py:111-122).  info: arena bytes, jobs, units, plans, table bytes
+ * moved by granule passes and by other passes with updates, kernel (1: the one with the fast forms of the
+ * others).  values: HOST uint32[nplans]. */
 void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, int *status);
 int tg_batch_info(void *batch, int64_t *info, int ninfo);
 /* window: plans in progress at once (0: all), admitted widest first */
@@ -285,6 +287,9 @@ int tg_server_submit(void *server, const int64_t *ops, int64_t nops);
 /* the same for a plan scheduled ahead of time by tg_dense_plan (uint8); the handle stays the caller's */
 int tg_server_submit_plan(void *server, void *plan);
 int tg_server_poll(void *server, int *slots, uint32_t *values, int max);
+/* the kernel that a launch for the plans now in progress takes (1: the one with the fast forms of other
+ * passes than granule passes) */
+int tg_server_form(void *server);
 int tg_server_stop(void *server);
 void tg_server_free(void *server);
 

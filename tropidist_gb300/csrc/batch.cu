@@ -112,6 +112,26 @@ __device__ void batch_single_op(const BJob &J, unsigned unit, const uint8_t *src
     }
 }
 
+// Table bytes that granule passes move, and that other passes with updates do: they choose the kernel.
+// Per GB of granule passes the spilling kernel takes 1.4 ms more (23 to 27 bits: 0.96 and 2.40 ms/GB) to 5.8
+// (14 to 20 bits); per GB of other passes the kernel without their fast forms takes 3.4 ms more (streaming
+// passes, 23 to 27 bits: 4.33 and 0.89 ms/GB) to 68 (14 to 20 bits), and 16 ms on 11-bit tiles.  The two are
+// even at 0.09 to 0.42 bytes of other passes per byte of granule passes: the line is drawn at a quarter.  A
+// plan under the default knobs has a stray other pass where two rows open or close at one column.
+struct PassWork {
+    double gran = 0, other = 0;
+    void add(const Seg &S) {
+        const double bytes = (double)((1ull << S.w_in) + (1ull << S.w_out));
+        if (S.kind == 4) gran += bytes;
+        else if (S.kind == 1 && S.pp.nupd > 0) other += bytes;
+    }
+    void add(const PassWork &o) {
+        gran += o.gran;
+        other += o.other;
+    }
+    bool take_fast() const { return 4 * other > gran; }
+};
+
 // steps of a granule pass by blocks of FP_THREADS threads
 __host__ __device__ __forceinline__ uint64_t gran_steps(const GranParams &P) {
     return (P.ncosets + FP_THREADS - 1) >> FP_TBITS;
@@ -166,9 +186,7 @@ static __device__ __noinline__ void fast_pass(const BJob &J, unsigned unit, cons
 
 // One unit of a job by the whole block; PRM = the block's copy of the job's parameters.  FAST: the passes
 // other than granule passes run in their fast forms.  A kernel that holds those (their register arrays,
-// a call) spills 4 KB a thread in the granule step, so the kernels come in both kinds and the one without
-// is used unless more than one pass in eight is of another form (a plan under the default knobs has a
-// stray one where two rows open or close at one column).
+// a call) spills 4 KB a thread in the granule step, so the kernels come in both kinds (take_fast).
 template <bool FAST>
 static __device__ __forceinline__ void run_unit(const BJob &J, unsigned unit, uint8_t *arena, const uint8_t *params,
                                                 uint4 *TC, uint4 *PRM) {
@@ -271,7 +289,7 @@ struct BatchPlan {
     std::vector<uint64_t> final_off;     // arena offset of each plan's final table
     std::vector<int> width;              // peak width of each plan
     uint64_t arena_bytes = 0;
-    int64_t ngran = 0, nother = 0;       // granule passes, other passes with updates
+    PassWork work;
     int64_t units = 0;
     void *dev = nullptr;                 // jobs, params, counters
     size_t dev_bytes = 0;
@@ -324,7 +342,7 @@ struct PlanJobs {
     int status = TG_OK;
     std::string error;
     int peak_bits = 0, final_buf = 0;
-    int64_t ngran = 0, nother = 0;
+    PassWork work;
     std::vector<BJob> jobs;
     std::vector<uint8_t> params;
 };
@@ -348,8 +366,7 @@ static void schedule_plan(const int64_t *ops, int64_t nops, PlanJobs &Q) {
                 Q.error = "batched plans need sweeps of <= 15 bits and tiles of <= 16 bits";
                 return;
             }
-            Q.ngran += S.kind == 4;
-            Q.nother += S.kind == 1 && S.pp.nupd > 0;
+            Q.work.add(S);
             BJob J;
             memset(&J, 0, sizeof(J));
             size_t bytes;
@@ -531,6 +548,7 @@ struct ServedPlan {
     uint64_t arena_off = 0, arena_bytes = 0, job0 = 0, njobs = 0, prm_off = 0, prm_bytes = 0;
     unsigned value = 0;
     unsigned tail_at_done = 0;     // queue tail read after the plan finished
+    PassWork work;
 };
 
 struct Server {
@@ -548,12 +566,18 @@ struct Server {
     std::vector<unsigned> free_slots;    // kept sorted, highest first: low slots are reused first
     unsigned mbox_tail = 0;
     int blocks = 0;
-    bool fast = false;                   // a plan with many passes of the other forms was admitted: launches from
-                                         // then on take the kernel that holds them (one that runs already
-                                         // takes such passes in their plain form)
     bool launched = false;
     unsigned *h_buf = nullptr;           // pinned: plan_done flags, then the control words
 };
+
+// the kernel for the plans in progress (one that runs already stays until its blocks idle out: it takes
+// other passes in their plain form, or granule passes with the spills)
+static bool server_fast(const Server &S) {
+    PassWork w;
+    for (const ServedPlan &R : S.plans)
+        if (R.live && !R.done) w.add(R.work);
+    return w.take_fast();
+}
 
 static int server_launch(Server &S) {
     if (S.launched && cudaStreamQuery(S.ks) == cudaErrorNotReady) return TG_OK;
@@ -580,7 +604,7 @@ static int server_launch(Server &S) {
         if (e) return e;
         attr = true;
     }
-    if (S.fast) k_server<true><<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
+    if (server_fast(S)) k_server<true><<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
     else k_server<false><<<S.blocks, BT_THREADS, BT_TILE_SMEM + 4096, S.ks>>>(A);
     S.launched = true;
     return cuda_check(cudaGetLastError(), "server launch");
@@ -621,8 +645,7 @@ void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, in
                 break;
             }
             B->width[i] = Q.peak_bits;
-            B->ngran += Q.ngran;
-            B->nother += Q.nother;
+            B->work.add(Q.work);
             const uint64_t tb = align_up((size_t)1 << Q.peak_bits, 256);
             const uint64_t a = B->arena_bytes, b = a + tb;
             B->arena_bytes = b + tb;
@@ -683,8 +706,9 @@ void *tg_batch_create(int nplans, const int64_t *ops, const int64_t *offsets, in
 int tg_batch_info(void *p, int64_t *info, int ninfo) {
     if (!p || !info) return set_error(TG_ERR_ARG, "null batch");
     const BatchPlan &B = *static_cast<BatchPlan *>(p);
-    int64_t v[4] = {(int64_t)B.arena_bytes, (int64_t)B.jobs.size(), B.units, B.nplans};
-    for (int k = 0; k < ninfo && k < 4; k++) info[k] = v[k];
+    int64_t v[7] = {(int64_t)B.arena_bytes, (int64_t)B.jobs.size(), B.units, B.nplans,
+                    (int64_t)B.work.gran, (int64_t)B.work.other, B.work.take_fast()};
+    for (int k = 0; k < ninfo && k < 7; k++) info[k] = v[k];
     return TG_OK;
 }
 
@@ -769,7 +793,7 @@ int tg_batch_run(void *p, void *arena, int blocks, int window, uint32_t *values,
     A.spin_limit = g_batch_spin ? g_batch_spin : 20000000ull;   // about 2.5 s of polling by default
     int grid = blocks > 0 ? blocks : sm_count();
     if (finished < (unsigned)B.nplans) {
-        if (8 * B.nother > B.ngran) k_batch<true><<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
+        if (B.work.take_fast()) k_batch<true><<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
         else k_batch<false><<<grid, BT_THREADS, BT_TILE_SMEM + 4096, st>>>(A);
         e = cuda_check(cudaGetLastError(), "batch launch");
         if (e) return e;
@@ -899,12 +923,7 @@ static int server_submit(Server &S, const DensePlan &P) {
         R.value = 0;
         return (int)slot;
     }
-    int64_t ngran = 0, nother = 0;
-    for (const Seg &G : P.segs) {
-        ngran += G.kind == 4;
-        nother += G.kind == 1 && G.pp.nupd > 0;
-    }
-    S.fast |= 8 * nother > ngran;
+    for (const Seg &G : P.segs) R.work.add(G);
     // parameter blob and jobs
     std::vector<uint8_t> prm;
     std::vector<BJob> jobs(P.segs.size());
@@ -1035,6 +1054,11 @@ int tg_server_poll(void *p, int *slots, uint32_t *values, int max) {
         }
     }
     return n;
+}
+
+int tg_server_form(void *p) {
+    if (!p) return set_error(TG_ERR_ARG, "null server");
+    return server_fast(*static_cast<Server *>(p)) ? 1 : 0;
 }
 
 // Makes the kernel's blocks leave and waits for them.
