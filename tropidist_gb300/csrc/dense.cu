@@ -356,6 +356,19 @@ static int g_span = 3, g_span_sel = 2;               // streaming passes: update
 // 4.74 / 2.15 ms; uint16 27 bits 10.9 / 1.73 ms.
 static bool use_gran(int eb) { return (eb == 1 ? g_dmax8 >= 12 : g_dmax16 >= 11) && g_span == 3 && g_span_sel == 2; }
 
+// Fewest ops between two kept tables (widest table of the interval: w bits) that granule passes take.  A
+// kept table is in canonical order, which the other forms write as they go where granule passes need a
+// pass of their own for it.  150 x 300 plans with a table kept every few ops, the two even at: uint8 9 ops
+// (17 bits; 6 % apart at most from 4 ops on), 6 (20), 7 (23), 8 to 9 (24), 8 to 10 (25), 10 (26), 12 (27), 17 (29),
+// 16 (30); uint16 9 (17), 7 to 8 (20, 23), 6 (24, 25), 6 (27), 6 to 7 (30).  At 27 bits uint8: every 4 ops
+// 2.85 ms with the other forms, 6.64 with granule passes; 8 ops 2.72, 3.73; 14 ops 2.42, 2.16.  A span whose end
+// table alone is kept (a plan that may end at any width) moves no copy of it: even at about 3/4 of that (uint8
+// 25 bits 6 to 7 ops, 27 bits 9, 29 bits 12; uint16 27 bits 4 to 5).
+static int gran_min_ops(int eb, int w) {
+    if (eb == 2) return w < 24 ? 9 : 6;
+    return w <= 17 ? 4 : w <= 24 ? 8 : std::min(16, 8 + 2 * (w - 24));
+}
+
 // Groups of the pass's updates whose chunk masks (mask >> 4) span <= 3 dimensions, every update
 // in a group (the in-chunk part of a mask is free in the register form; see fused_u8.cuh).  Also
 // the thread -> coset maps and the store mode.  use_groups = 0 when the register form does not
@@ -755,9 +768,7 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
     const int DMAX = eb == 1 ? g_dmax8 : g_dmax16;
     const int SWB = eb == 1 ? g_sweep_bits8 : g_sweep_bits16;
     const bool relayout = eb == 1 && g_relayout;
-    // a table kept after every op or two (a leaf of the witness traceback) leaves a granule pass one column:
-    // the other forms need no reordering there (26-bit witness: 156 ms, 209 with granule passes in the leaves)
-    const bool gran = use_gran(eb) && nops >= 4 * nckpt;
+    const bool gran_on = use_gran(eb);
     P.eb = eb;
     P.peak_bits = peak;
     P.nops = nops;
@@ -958,6 +969,20 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
     // the first checkpoint after each op (nops when none)
     std::vector<int64_t> next_ckpt(nops + 2, nops);
     for (int64_t k = nops - 1; k >= 0; k--) next_ckpt[k] = is_ckpt[k + 1] ? k + 1 : next_ckpt[k + 1];
+    // granule passes in the interval from op i0 (a kept table or the start, of width w) to the next kept table?
+    auto take_gran = [&](int64_t i0, int w) {
+        const int64_t end = next_ckpt[i0];
+        const bool kept = end < nops;
+        if (!gran_on || !(kept || open_end)) return gran_on;
+        int widest = w;
+        for (int64_t k = i0; k < end && k < i0 + 16; k++) {
+            w += hops[k].code == 0 ? 1 : hops[k].code == 2 ? -1 : 0;
+            widest = std::max(widest, w);
+        }
+        const int need = gran_min_ops(eb, widest);
+        return end - i0 >= (kept ? need : 3 * need / 4);
+    };
+    bool gran = false;
     // scratch of the pass-growing loop (assigned per candidate op, no allocation once grown)
     std::vector<int> t2, cur2, need;
     std::vector<uint64_t> b2;
@@ -968,6 +993,7 @@ int build_dense_plan(const int64_t *ops, int64_t nops, int eb, const int64_t *ck
     while (i < nops) {
         const int w_in = (int)canon.size();
         const int64_t limit = next_ckpt[i];
+        if (i == 0 || is_ckpt[i]) gran = take_gran(i, w_in);
         Seg S;
         S.w_in = w_in;
         const int64_t i_seg = i;
