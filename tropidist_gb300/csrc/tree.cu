@@ -333,6 +333,7 @@ __global__ void __launch_bounds__(TR_BS, 3) k_tree_join(const TJoin *joins, int 
 #define TG_T 64
 #define TG_KC 32
 #define TG_LD (TG_T + 4)
+#define TG_MAXKB 15                    // 2^kb products are the grid's z, which holds at most 65535
 
 struct TGemm {
     int64_t lo, ro, po;                // arena offsets of the left, right and parent tables
@@ -679,7 +680,7 @@ void *tg_tree_plan(const int64_t *leaves, int64_t nleaves, const int64_t *joins,
         const int64_t j = r[0], F = r[1] & 255, rows = r[1] >> 8, mb = r[2], nb = r[3], kb = r[4], mo = r[5];
         const int64_t nm = rows ? 3 * (mb + nb) + 4 * kb : 2 * (mb + nb + kb);
         if (rows < 0 || rows > 1 || j < 0 || j >= njoins || gemm_of[j] >= 0 || F < 2 || F > 30 || mb < 6 || mb > 21 ||
-            nb < 6 || nb > 21 || kb < 0 || kb > 16 || mo < 0 || mo + nm > ngmaps || hj[j].F != F ||
+            nb < 6 || nb > 21 || kb < 0 || kb > TG_MAXKB || mo < 0 || mo + nm > ngmaps || hj[j].F != F ||
             hj[j].P != mb + nb + kb) {
             st = set_error(TG_ERR_ARG, "bad tree gemm row");
             break;

@@ -481,7 +481,7 @@ class CompiledTreeDP:
             for i in by_h[h]:
                 nd, jn = self.nodes[i], self.joins[i]
                 g = gemm_form(jn)
-                if g is not None and g["F"] >= 2 and 6 <= g["mb"] <= 21 and 6 <= g["nb"] <= 21 and g["kb"] <= 16:
+                if g is not None and runs_as_product(g):
                     grows.append([len(rows), g["F"] | GEMM_ROWS, g["mb"], g["nb"], g["kb"], len(gmaps)])
                     for k in ("DL", "DR", "DT", "PA", "PB", "PT", "GA", "GB", "TA", "TB"):
                         gmaps.extend(g[k])
@@ -703,6 +703,12 @@ def gemm_form(join):
     return {"F": F, "mb": len(PA), "nb": len(PB), "kb": len(PT), "PA": PA, "PB": PB, "PT": PT,
             "DL": [d_of(c) for c in PA], "DR": [d_of(c) for c in PB], "DT": [d_of(c) for c in PT],
             "GA": GA, "GB": GB, "TA": TA, "TB": TB}
+
+
+def runs_as_product(g):
+    """Does the device run this block-product form (tg_tree_plan)?  At least 64 rows a side and rows of 4
+    entries; at most 2^15 tiles of left rows and 2^15 products, the limits of a launch grid."""
+    return g["F"] >= 2 and 6 <= g["mb"] <= 21 and 6 <= g["nb"] <= 21 and g["kb"] <= 15
 
 
 def _vanishing(vectors, part):
