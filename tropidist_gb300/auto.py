@@ -15,13 +15,15 @@ import time
 
 from . import kernel, trellis
 
-# state-updates per second of the GPU executor, for predictions only (measured on GB300 with the
-# fused passes; tables narrower than ~20 bits are launch-bound and slower)
-RATE_GPU = 5.0e12
+# State-updates per second of the GPU executor, for predictions only: wide sweeps, and the fit of one
+# observable's sweep by its peak width (uint8, 1000 x 2000 banded plans: 1.18e13 at 31 bits, 1.04e13 at 30,
+# 8.1e12 at 28, 2.8e12 to 5.3e12 at 26, 1.1e12 at 24, 2.8e11 at 22, 1.7e10 to 3.2e10 at 19: narrow passes
+# are bound by their launch and latency, so their rate halves with every bit).
+RATE_GPU = 1.2e13
 
 
 def predicted_seconds(work, width=30):
-    rate = RATE_GPU if width >= 22 else RATE_GPU * 2.0 ** (width - 22)
+    rate = RATE_GPU / (1.0 + 2.0 ** (27 - width))
     return work / max(rate, 1e9)
 
 
