@@ -352,7 +352,8 @@ static int g_span = 3, g_span_sel = 2;               // streaming passes: update
                                                      // span when an in-chunk row closes in the pass
 // Granule passes take the wide tables of both entry sizes unless a knob asks for another form: a tile
 // narrower than the 2^12 bytes that a warp of the granule pass holds, or a streaming span other than
-// the default.  One sweep, the other forms against granule passes: uint8 31 bits 48.4 / 19.2 ms, 26 bits
+// the default.  They hold at most 2^32 granules (gran_sched.h), and not every interval between kept tables is
+// worth one (gran_min_ops).  One sweep, the other forms against granule passes: uint8 31 bits 48.4 / 19.2 ms, 26 bits
 // 4.74 / 2.15 ms; uint16 27 bits 10.9 / 1.73 ms.
 static bool use_gran(int eb) { return (eb == 1 ? g_dmax8 >= 12 : g_dmax16 >= 11) && g_span == 3 && g_span_sel == 2; }
 

@@ -15,15 +15,16 @@
 //   A  column that opens a row and closes another: the new row takes the old one's place, w is added
 //      where the new row is 1; no slot at all;
 //   T  the row of a slot changes places with an in-granule row (a register transposition).
-// So a pass of 5 slots takes 8 to 10 columns of a banded plan, where a pass that keeps the opened
-// rows' INF halves and the closed rows' dropped halves in its registers takes 2 to 3.
+// So a pass of 5 slots takes 7.3 columns of the 31-bit banded plan on average (6 to 8 in its widest
+// passes), where a pass that keeps the opened rows' INF halves and the closed rows' dropped halves in its
+// registers takes 2 to 3.
 //
 // A warp's lanes are the lowest coset-number bits, which are the lowest input positions that no
 // member direction uses, and the output order keeps the lowest three of them low: a warp reads and
 // writes whole 32-byte sectors (usually 128-byte lines) with 4-byte accesses, so the table needs no
 // shared-memory staging.
 //
-// Bound: issue slots (VIADDMNMX, LOP3 and the address arithmetic; 62-70 % of the issue rate, the ALU pipe
+// Bound: issue slots (VIADDMNMX, LOP3 and the address arithmetic; 60-68 % of the issue rate on tables of 2^27 to 2^30 entries, the ALU pipe
 // next), not HBM: on the 31-bit plan (window 37) a sweep moves 57 GB in 270 passes where the
 // chunk-streaming passes moved 181 GB in 735, and takes 19.2 ms instead of 47.2 ms; 26 bits 2.15 instead
 // of 4.74 ms; uint16 at 27 bits 1.73 instead of 10.9 ms (tile passes).

@@ -7,7 +7,12 @@ namespace tg {
 
 #define GP_MINW 9            // narrowest table of a pass (input and output)
 #define GP_MAXBITS 32        // widest, in granules: the kernel's offsets are 32-bit granule numbers
-#define GP_EVICT_OPS 40      // an in-granule row that closes within this many ops leaves the granule
+// An in-granule row that closes within GP_EVICT_OPS ops leaves the granule, for a row that lives GP_EVICT_GAIN
+// ops longer at least.  A 300 x 600 sweep at 10 / 20 / 40 / 80 / 160 ops: uint8 30 bits 5.93 / 3.93 / 3.68 /
+// 3.74 / 4.09 ms, 26 bits 0.81 / 0.76 / 0.74 / 0.75 / 0.76; uint16 26 bits 1.10 / 1.02 / 1.01 / 0.95 / 0.94.
+// The gain: 1, 8, 16 and 32 within 2 % of each other, 64 5 % slower at 30 bits (a row stays that should leave).
+#define GP_EVICT_OPS 40
+#define GP_EVICT_GAIN 16
 
 // value of a row as a parity of register slots, coset-number bits and a constant
 struct RowExpr {
@@ -73,7 +78,7 @@ static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, in
         int best = -1;
         for (int p = G + 3; p < w_in; p++)
             if ((best < 0 || life(p) > life(best)) && !(nsw && sw[0].row == p)) best = p;
-        if (best < 0 || (life(best) != INT64_MAX && life(best) < life(g) + 16)) continue;
+        if (best < 0 || (life(best) != INT64_MAX && life(best) < life(g) + GP_EVICT_GAIN)) continue;
         sw[nsw++] = {g, best, -1};
         insert(1ull << best);
         L++;
@@ -388,7 +393,7 @@ static int64_t build_gran(const std::vector<HostOp> &hops, const RowInfo &RI, in
     return j;
 }
 
-// the granule pass on host memory, coset by coset, entry by entry (gran_range's maps and program)
+// the granule pass on host memory, coset by coset, entry by entry (gran_step's maps and program)
 template <typename E>
 static void emulate_gran(const GranParams &P, const E *src, E *dst) {
     constexpr int EB = sizeof(E), NE = 4 / EB;            // entries per granule
