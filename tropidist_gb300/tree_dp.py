@@ -480,7 +480,9 @@ class CompiledTreeDP:
         for h in range(1, H + 1):
             for i in by_h[h]:
                 nd, jn = self.nodes[i], self.joins[i]
-                g = gemm_form(jn)
+                # a tree with a wider table is accounted for here and does not run
+                narrow = max(jn.left_rank, jn.right_rank, jn.parent_rank) <= DEVICE_INDEX_BITS
+                g = gemm_form(jn) if narrow else None
                 if g is not None and runs_as_product(g):
                     grows.append([len(rows), g["F"] | GEMM_ROWS, g["mb"], g["nb"], g["kb"], len(gmaps)])
                     for k in ("DL", "DR", "DT", "PA", "PB", "PT", "GA", "GB", "TA", "TB"):
