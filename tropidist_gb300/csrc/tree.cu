@@ -329,7 +329,8 @@ __global__ void __launch_bounds__(TR_BS, 3) k_tree_join(const TJoin *joins, int 
 // A tile reads a child entry once for 64 pairs where the per-pair kernel reads two entries a pair: a
 // 240-column tree with joins of 2^31 to 2^33 pairs takes 2.35 ms for 4 targets, 4.65 ms with products
 // only where every block meets every other.  Joins of fewer than 64 rows on a side or of F < 2 stay
-// with the per-pair kernel (2^22 pairs at most on such trees).
+// with the per-pair kernel (2^22 pairs at most on such trees), and so do those with couplings and fewer
+// than 2^22 pairs (measured beside worth_a_product in tree_dp.py).
 #define TG_T 64
 #define TG_KC 32
 #define TG_LD (TG_T + 4)

@@ -483,7 +483,7 @@ class CompiledTreeDP:
                 # a tree with a wider table is accounted for here and does not run
                 narrow = max(jn.left_rank, jn.right_rank, jn.parent_rank) <= DEVICE_INDEX_BITS
                 g = gemm_form(jn) if narrow else None
-                if g is not None and runs_as_product(g):
+                if g is not None and runs_as_product(g) and worth_a_product(jn, g):
                     grows.append([len(rows), g["F"] | GEMM_ROWS, g["mb"], g["nb"], g["kb"], len(gmaps)])
                     for k in ("DL", "DR", "DT", "PA", "PB", "PT", "GA", "GB", "TA", "TB"):
                         gmaps.extend(g[k])
@@ -711,6 +711,20 @@ def runs_as_product(g):
     """Does the device run this block-product form (tg_tree_plan)?  At least 64 rows a side and rows of 4
     entries; at most 2^15 tiles of left rows and 2^15 products, the limits of a launch grid."""
     return g["F"] >= 2 and 6 <= g["mb"] <= 21 and 6 <= g["nb"] <= 21 and g["kb"] <= 15
+
+
+# A product is a launch of its own (some 10 us on the path of the tree's heights), where the per-pair kernel
+# takes all joins of a height in one.  Trees of 90 to 400 columns (window 8 to 13) by the fewest pairs of a coupled
+# join's product (log2), against no coupled products at all: 16 0.82 of the time (1.27 on the worst tree), 18 0.80
+# (1.09), 20 0.79 (1.07), 21 0.79 (1.05), 22 0.80 (1.01), 23 0.83 (1.00), 24 0.88 (1.00).
+COUPLED_PRODUCT_BITS = 22
+
+
+def worth_a_product(join, g):
+    """Is the form faster than the per-pair kernel?  Where every left block meets every right block, yes; with
+    couplings from 2^22 pairs on."""
+    onto = g["mb"] + g["nb"] == join.left_rank + join.right_rank - 2 * g["F"]
+    return onto or join.parent_rank + g["F"] >= COUPLED_PRODUCT_BITS
 
 
 def _vanishing(vectors, part):
