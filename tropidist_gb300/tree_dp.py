@@ -480,9 +480,11 @@ class CompiledTreeDP:
         for h in range(1, H + 1):
             for i in by_h[h]:
                 nd, jn = self.nodes[i], self.joins[i]
-                # a tree with a wider table is accounted for here and does not run
+                # no form is looked for where it could not run: fewer than 64 rows a side, rows of fewer than 4
+                # entries, or a wider table (its tree is accounted for here, and refused)
+                F = len(jn.free_maps)
                 narrow = max(jn.left_rank, jn.right_rank, jn.parent_rank) <= DEVICE_INDEX_BITS
-                g = gemm_form(jn) if narrow else None
+                g = gemm_form(jn) if narrow and F >= 2 and min(jn.left_rank, jn.right_rank) >= F + 6 else None
                 if g is not None and runs_as_product(g) and worth_a_product(jn, g):
                     grows.append([len(rows), g["F"] | GEMM_ROWS, g["mb"], g["nb"], g["kb"], len(gmaps)])
                     for k in ("DL", "DR", "DT", "PA", "PB", "PT", "GA", "GB", "TA", "TB"):
