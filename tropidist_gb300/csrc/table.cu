@@ -15,6 +15,7 @@
 #include "tg_common.cuh"
 #include "tg_capi.h"
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -63,10 +64,12 @@ __global__ void k_tb_clear(unsigned long long *keys, uint64_t nwords, uint8_t *c
 }
 
 // Bound by the latency of a slot's random access: the claim goes straight to the compare-and-swap (half
-// the slots or more are empty, so a load before it is a second round trip), and a thread counts the keys
+// the slots or more are empty, so a load before it is a second round trip) unless most subsets meet a key
+// that is there already (LOOK, tb_few_keys: a compact slot is read first), and a thread counts the keys
 // it created and adds them once per warp (an add per key on the one counter serialised the launch).
 // C(301, 3) subsets into 2^24 slots with their lookup: 1.26 ms a pass, 1.52 before; the 1 + 169 + 14196
 // subsets of a distance-13 search: 47 us in all, 94 before.
+template <bool LOOK>
 __global__ void k_tb_build(TableHandle T, int s, uint64_t nsub, int n, const unsigned long long *binom,
                            const unsigned long long *zh, const unsigned long long *zl, const unsigned long long *lg,
                            unsigned long long *errflag) {
@@ -82,7 +85,8 @@ __global__ void k_tb_build(TableHandle T, int s, uint64_t nsub, int n, const uns
         if (!T.wide) {
             const uint64_t key = tb_compact_key(l, g);
             for (uint64_t probe = 0; probe <= mask && !done; probe++) {
-                const unsigned long long prev = atomicCAS(T.keys + i, 0ull, (unsigned long long)key);
+                unsigned long long prev = LOOK ? T.keys[i] : 0ull;
+                if (prev == 0ull) prev = atomicCAS(T.keys + i, 0ull, (unsigned long long)key);
                 if (prev == 0ull) {
                     T.cost[i] = (uint8_t)s;
                     created++;
@@ -114,6 +118,24 @@ __global__ void k_tb_build(TableHandle T, int s, uint64_t nsub, int n, const uns
     }
     created = __reduce_add_sync(0xffffffffu, created);
     if ((threadIdx.x & 31) == 0 && created) atomicAdd(T.count, (unsigned long long)created);
+}
+
+// Do the subsets of n columns share few compact keys?  Keys are sums of the columns' (fingerprint, label)
+// pairs: at most 2^rank of them.  Compare-and-swaps on few keys queue up where loads do not (C(300, 3)
+// subsets, swaps alone against a load first: 2^6 keys 1.36 and 0.16 ms, 2^10 0.33 and 0.16, 2^16 0.183 and 0.167,
+// 2^22 0.211 and 0.204, 2^30 0.280 and 0.282; C(100, 3): 2^8 66 and 53 us, 2^12 55 and 55, 2^18 56 and 68; C(400, 2):
+// 2^8 53 and 52, 2^10 48 and 52): from 128 subsets a key on, in tables of 2^20 subsets and more from 32.
+static bool tb_few_keys(int n, const uint64_t *zl, const uint64_t *lg, uint64_t total) {
+    const int per = total >> 20 ? 5 : 7;
+    std::vector<unsigned __int128> basis;                // distinct top bits, descending
+    for (int j = 0; j < n; j++) {
+        unsigned __int128 v = ((unsigned __int128)(zl[j] & TB_FPMASK) << 16) | (lg[j] & 0xFFFFull);
+        for (const unsigned __int128 b : basis) v = std::min(v, v ^ b);
+        if (!v) continue;
+        if (((uint64_t)1 << (basis.size() + 1 + per)) > total) return false;
+        basis.insert(std::find_if(basis.begin(), basis.end(), [v](unsigned __int128 b) { return b < v; }), v);
+    }
+    return total >> per != 0;
 }
 
 __global__ void k_tb_lookup(TableHandle T, uint64_t m, const unsigned long long *zh, const unsigned long long *zl,
@@ -295,14 +317,18 @@ int tg_tab_build(void *p, int n, const uint64_t *zh, const uint64_t *zl, const u
         memcpy(h + nb + nh, zl, (size_t)n * 8);
         memcpy(h + nb + 2 * nh, lg, (size_t)n * 8);
     }
+    uint64_t total = 0;
+    for (int s = 0; s <= k; s++) total += binom[(uint64_t)n * (TB_MAXK + 1) + s];
     memset(h + nb + 3 * nh, 0, 8);
     unsigned long long *dbin = d, *dzh = d + binom.size(), *dzl = dzh + std::max(n, 1), *dlg = dzl + std::max(n, 1);
     unsigned long long *derr = dlg + std::max(n, 1);
     cudaStream_t st = 0;
+    const bool look = !T->wide && tb_few_keys(n, zl, lg, total);
     int e = cuda_check(cudaMemcpyAsync(d, h, tot, cudaMemcpyHostToDevice, st), "build inputs");
     for (int s = 0; s <= k && !e; s++) {
         const uint64_t nsub = binom[(uint64_t)n * (TB_MAXK + 1) + s];
-        k_tb_build<<<tb_grid(nsub), 256, 0, st>>>(*T, s, nsub, n, dbin, dzh, dzl, dlg, derr);
+        if (look) k_tb_build<true><<<tb_grid(nsub), 256, 0, st>>>(*T, s, nsub, n, dbin, dzh, dzl, dlg, derr);
+        else k_tb_build<false><<<tb_grid(nsub), 256, 0, st>>>(*T, s, nsub, n, dbin, dzh, dzl, dlg, derr);
         e = cuda_check(cudaGetLastError(), "table build");
     }
     unsigned long long *hr = reinterpret_cast<unsigned long long *>(h);
